@@ -394,12 +394,16 @@ int gol_init(gol_engine* e) {
         }
     }
     int k = (int)e->cfg.temporal_steps;
-    // Auto depth: 4 (the dense optimum on B200); 6 with change tracking,
-    // where a pass of k generations sees oscillators whose period divides k
-    // as still (period 2 blinkers and period 3 pulsars are most of the ash
-    // a random grid settles into).
-    if (k <= 0) k = e->cfg.algorithm == GOL_ALG_LOCAL ? 6 : 4;
     const int sms = golb200::device_sm_count(e->cfg.device);
+    // Auto depth: where a generation costs least on this grid; with a forced
+    // band or lane width 4, the K-stage kernel's optimum; 6 with change
+    // tracking, where a pass of k generations sees oscillators whose period
+    // divides k as still (period 2 blinkers and period 3 pulsars are most of
+    // the ash a random grid settles into).
+    if (k <= 0)
+        k = e->cfg.algorithm == GOL_ALG_LOCAL                    ? 6
+            : e->cfg.thread_block_size || e->cfg.lane_words ? 4
+                                                            : golb200::best_depth(e->W, e->Y, sms);
     if (!golb200::plan_rows(e->W, e->Y, k, (int)e->cfg.thread_block_size,
                             (int)e->cfg.lane_words, sms, &e->plan))
         return e->fail(GOL_E_UNSUPPORTED, "no kernel plan for this width and depth");

@@ -25,15 +25,21 @@ struct RowsPlan {
     int halo = 0;      // x-halo words each side of a slice (0 when unsliced)
     bool stream = false;   // k = 1 streaming kernel (gol_rows_stream.cuh): band = rows
                            // per thread, nslices = CTAs across the row, no halo
+    int block = 0;         // register-block kernel (gol_rows_block.cuh): R, the rows a warp
+                           // holds; band = rows it stores, nbands = blocks of rows
 };
 
 // Picks words-per-lane and CTA shape for a W-word by Y-row grid and depth k.
 // wpl = 0 chooses the widest lane access whose rings fit k; 1, 2 or 4 forces
 // it. Returns false for k outside 1..16 or a wpl that W or k rules out.
 // k = 1 plans the streaming kernel (band_rows = rows per thread, 0 = auto)
-// unless allow_stream is false (callers that need the K-stage geometry).
+// and deeper passes without a forced band or wpl the register-block kernel
+// unless k_stage is set (callers that need the K-stage geometry).
 bool plan_rows(int W, int Y, int k, int band_rows, int wpl, int num_sms, RowsPlan* plan,
-               bool allow_stream = true);
+               bool k_stage = false);
+
+// The depth at which a generation of a W-word by Y-row grid costs least.
+int best_depth(int W, int Y, int num_sms);
 
 // Shared-memory-resident run (gol_rows_resident.cuh): every generation of
 // a grid whose bands fit in the SMs' shared memory, in one cooperative

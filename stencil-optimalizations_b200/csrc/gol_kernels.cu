@@ -1,9 +1,11 @@
 // Kernel instantiations and launch dispatch for the row-band temporal
 // kernel, plus device-side pack/unpack between uint8 cells and row words.
 #include <algorithm>
+#include <cmath>
 
 #include "gol_b200.h"
 #include "gol_internal.h"
+#include "gol_rows_block.cuh"
 #include "gol_rows_resident.cuh"
 #include "gol_rows_stream.cuh"
 #include "gol_rows_temporal.cuh"
@@ -67,6 +69,53 @@ cudaError_t launch_stream(const RowsLaunch& a, const RowsPlan& p, cudaStream_t s
     return cudaLaunchKernelEx(&cfg, rows_stream_kernel<WPL>, a);
 }
 
+// The register-block kernel, a programmatic dependent too.
+template <int R>
+cudaError_t launch_block(const BlockLaunch& a, cudaStream_t stream) {
+    const long long warps = ((long long)a.nblocks * (a.W + 1) + kBlockOwn - 1) / kBlockOwn;
+    if (warps > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)warps);
+    cfg.blockDim = dim3(32);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, rows_block_kernel<R>, a);
+}
+
+// Estimated time (us) of a register-block pass and its best block. Fitted to
+// passes at 256^2 .. 16384^2, K = 4 and 8, to about 10 %: a warp takes
+// `rows` row-generations (plus about 2.5 a generation for the exits every
+// four rows and the first two rows' sums) at 28.5 cycles each when it has its
+// scheduler to itself, 25.5 beside one other and 23.5 beside more (the
+// integer pipe alone: 20), a few cycles a row for loads and stores, and a
+// pass a fixed part for its launch and first loads. Short blocks waste rows,
+// tall ones leave schedulers idle, so the block's height is searched.
+struct BlockChoice {
+    int R = 0, B = 0;
+    double us = 0;
+};
+
+BlockChoice best_block(int W, int Y, int k, int num_sms) {
+    BlockChoice best;
+    for (int R : {32, 48, 64, 96}) {
+        for (int B = std::min(R - 2 * k, (Y + 1) / 2 * 2); B >= 2; B -= B > 4 ? 4 : 2) {
+            const long long nblocks = ((long long)Y + B - 1) / B;
+            const double warps = (double)(nblocks * (W + 1)) / kBlockOwn;
+            double n = warps / (4.0 * num_sms);   // warps per scheduler
+            if (n < 8) n = std::ceil(n);
+            const double cycles = n <= 1 ? 28.5 : n <= 2 ? 25.5 : 23.5;
+            const double rows = (double)k * (B + k - 1 + 2.5);
+            const double us = 0.9 + 0.018 * R + n * (0.0083 * R + rows * cycles / 1965.0);
+            if (!best.R || us < best.us) best = {R, B, us};
+        }
+    }
+    return best;
+}
+
 template <int WPL, int K>
 cudaError_t dispatch_k(int k, const RowsLaunch& a, const RowsPlan& p, cudaStream_t stream) {
     if constexpr (K > kMaxKForWpl(WPL)) {
@@ -85,9 +134,23 @@ int device_sm_count(int device) {
     return n > 0 ? n : 148;
 }
 
+int best_depth(int W, int Y, int num_sms) {
+    int best = 4;
+    double t = 0;
+    for (int k : {4, 6, 8, 12, 16}) {
+        const double u = best_block(W, std::max(Y, 1), k, num_sms).us / k;
+        if (t == 0 || u < t) {
+            t = u;
+            best = k;
+        }
+    }
+    return best;
+}
+
 bool plan_rows(int W, int Y, int k, int band_rows, int wpl, int num_sms, RowsPlan* plan,
-               bool allow_stream) {
+               bool k_stage) {
     if (k < 1 || k > kMaxTemporalSteps || W <= 0) return false;
+    const bool forced = wpl != 0 || band_rows > 0;
     if (wpl != 0) {
         if ((wpl != 1 && wpl != 2 && wpl != 4) || W % wpl || k > kMaxKForWpl(wpl)) return false;
     } else {
@@ -102,7 +165,20 @@ bool plan_rows(int W, int Y, int k, int band_rows, int wpl, int num_sms, RowsPla
     }
     plan->wpl = wpl;
     const int lanes = W / wpl;
-    plan->stream = k == 1 && allow_stream;
+    plan->stream = k == 1 && !k_stage;
+    plan->block = 0;
+    if (k > 1 && !k_stage && !forced) {
+        const BlockChoice c = best_block(W, std::max(Y, 1), k, num_sms);
+        plan->wpl = 1;
+        plan->threads = 32;
+        plan->block = c.R;
+        plan->band = c.B;
+        plan->nbands = (int)(((long long)Y + c.B - 1) / c.B);
+        plan->slice = kBlockOwn;
+        plan->nslices = (W + kBlockOwn - 1) / kBlockOwn;
+        plan->halo = 1;
+        return true;
+    }
     if (plan->stream) {
         // One generation: lanes of wpl words across the row in CTAs of up to
         // GOL_STREAM_THREADS threads, each thread walking `band` rows. The
@@ -242,6 +318,17 @@ cudaError_t launch_resident(const uint32_t* src, uint32_t* dst, int W, int Y, lo
 cudaError_t launch_rows_pass(const uint32_t* src, uint32_t* dst, int W, int Y, int k,
                              const RowsPlan& p, cudaStream_t stream, int pitch) {
     if (Y <= 0 || W <= 0) return cudaSuccess;
+    if (p.block) {
+        if (k < 1 || p.band + 2 * k > p.block) return cudaErrorInvalidValue;
+        const BlockLaunch b{src, dst, W, Y, pitch ? pitch : W, p.band, k, p.nbands};
+        switch (p.block) {
+            case 32: return launch_block<32>(b, stream);
+            case 48: return launch_block<48>(b, stream);
+            case 64: return launch_block<64>(b, stream);
+            case 96: return launch_block<96>(b, stream);
+            default: return cudaErrorInvalidValue;
+        }
+    }
     RowsLaunch a{src, dst, W, Y, p.band, p.slice, p.halo, pitch ? pitch : W};
     if (p.stream) {
         if (k != 1) return cudaErrorInvalidValue;

@@ -1,0 +1,126 @@
+// Register-block pass: K generations of a block of rows held in registers.
+//
+// One warp advances 32 adjacent words of a row by R rows (R a compile-time
+// constant): each lane keeps its word of every row in a register, loaded
+// once, advanced K generations in place and stored once. There is no shared
+// memory and no barrier, and the rows of a generation are independent of
+// each other, so a warp alone keeps its scheduler three quarters busy. What
+// bounds it is the integer pipe: ten operations per word and generation
+// (two shifts, two for the horizontal sum, six for the rule, which two rows
+// at a time share; gol_word_ops.cuh).
+//
+//   * Rows: a block of B output rows loads B + 2K rows; each generation the
+//     rows still correct shrink by one at either end (about 9 % more rows
+//     computed than stored at K = 8, R = 96). Generation g writes row i to
+//     register i - 1, so the rows that count always start at register 0:
+//     one loop body serves every generation and every K, leaving early once
+//     the rows that still count are done.
+//   * Columns: the words beyond a lane's own come from its neighbours by
+//     shuffle. The outer two lanes are context (errors from the words beyond
+//     them move one cell per generation and stay inside them for K <= 32),
+//     so a warp stores 30 of its 32 columns.
+//   * A row's columns need not be a multiple of 30: the columns of all blocks
+//     of rows stand in one line, a dead column after each row, and warp w
+//     takes columns 30 w - 1 .. 30 w + 30 of it, each lane in its own block.
+//     Only warps that hold a dead column, or rows outside the grid, mask
+//     their words after each generation.
+//   * One warp per CTA, and the next pass is let in only when the block is
+//     about to be stored: passes are programmatic dependents, and CTAs of the
+//     next pass that became resident earlier took the place of this pass's
+//     on some SMs (8.2 against 11.3 us per pass of 8 generations at
+//     5024 x 3001, R = 32, B = 16).
+// Measured (K = 8): 16384^2 58.3 us per pass (36.8 T cell-updates/s, R = 96,
+// B = 80), 10240 x 6001 18.5 us (55.6 for the K-stage kernel of
+// gol_rows_temporal.cuh), 5024 x 3001 7.6 us (two K-stage passes of 4: 20.8),
+// 2048^2 4.4 us.
+#pragma once
+
+#include <cstdint>
+
+#include "gol_rows_temporal.cuh"
+#include "gol_word_ops.cuh"
+
+namespace golb200 {
+
+constexpr int kBlockOwn = 30;   // columns a warp stores
+
+struct BlockLaunch {
+    const uint32_t* src;   // gen-0 grid (row r at src + r * pitch)
+    uint32_t* dst;         // gen-K grid (must not alias src)
+    int W, Y, pitch;
+    int B;                 // rows stored per block (even, B + 2K <= R)
+    int K;
+    int nblocks;           // blocks of rows
+};
+
+template <int R>
+constexpr int block_min_ctas() { return R <= 32 ? 32 : R <= 48 ? 24 : R <= 64 ? 20 : 16; }
+
+// Horizontal sum of this lane's word of one row (bit planes 0 and 1).
+__device__ __forceinline__ void block_hsum(uint32_t c, uint32_t& h0, uint32_t& h1) {
+    const uint32_t lw = __shfl_up_sync(0xffffffffu, c, 1);
+    const uint32_t rw = __shfl_down_sync(0xffffffffu, c, 1);
+    hsum(lw, c, rw, h0, h1);
+}
+
+template <int R>
+__global__ void __launch_bounds__(32, block_min_ctas<R>()) rows_block_kernel(BlockLaunch a) {
+    static_assert(R % 4 == 0, "rows are taken two at a time, the exit tested every four");
+    const int lane = threadIdx.x;
+    const long long line = a.W + 1;
+    const long long idx = (long long)blockIdx.x * kBlockOwn - 1 + lane;
+    const int block = idx < 0 ? 0 : (int)(idx / line);
+    const int col = (int)(idx - block * line);   // -1: before the first column, W: a dead column
+    const bool ok = idx >= 0 && block < a.nblocks && col < a.W;
+    const int y0 = block * a.B - a.K;            // row of w[0]
+    const bool inside = __all_sync(0xffffffffu, ok && y0 >= 0 && y0 + R <= a.Y);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    uint32_t w[R];
+    const uint32_t* p = a.src + (long long)y0 * a.pitch + col;   // dereferenced inside the grid only
+    if (inside) {
+#pragma unroll
+        for (int r = 0; r < R; ++r, p += a.pitch) w[r] = __ldg(p);
+    } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r, p += a.pitch)
+            w[r] = ok && (unsigned)(y0 + r) < (unsigned)a.Y ? __ldg(p) : 0u;
+    }
+    for (int g = 1; g <= a.K; ++g) {
+        const int n = a.B + 2 * (a.K - g);   // rows that count after this generation
+        uint32_t a0, a1, b0, b1;
+        block_hsum(w[0], a0, a1);
+        block_hsum(w[1], b0, b1);
+#pragma unroll
+        for (int j = 0; j + 3 < R; j += 2) {   // rows j + 1 and j + 2 of the block
+            if (j % 4 == 0 && j >= 8 && j >= n) break;
+            uint32_t p0, p1, q0, q1;
+            block_hsum(w[j + 2], p0, p1);
+            block_hsum(w[j + 3], q0, q1);
+            const PairSum s = pair_sum(b0, b1, p0, p1);
+            const uint32_t up = next_word_pair(a0, a1, s, w[j + 1]);
+            const uint32_t down = next_word_pair(q0, q1, s, w[j + 2]);
+            w[j] = up;
+            w[j + 1] = down;
+            a0 = p0;
+            a1 = p1;
+            b0 = q0;
+            b1 = q1;
+        }
+        if (!inside) {   // columns and rows outside the grid stay dead
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                w[r] = ok && (unsigned)(y0 + g + r) < (unsigned)a.Y ? w[r] : 0u;
+        }
+    }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (ok && lane >= 1 && lane <= kBlockOwn) {
+        const int ys = block * a.B;
+        const int rows = min(a.B, a.Y - ys);
+        uint32_t* d = a.dst + (long long)ys * a.pitch + col;
+#pragma unroll
+        for (int r = 0; r < R - 2; ++r, d += a.pitch)
+            if (r < rows) *d = w[r];
+    }
+}
+
+} // namespace golb200
