@@ -24,6 +24,8 @@ thread_local std::string g_create_error;
 // Passes per captured CUDA graph (even, so a chunk ends on the same buffer
 // parity it started from and one executable graph per parity suffices).
 constexpr int kGraphPasses = 16;
+constexpr int kLocalGraphPasses = 18;
+static_assert(kLocalGraphPasses % golb200::kLocalPhases == 0, "a chunk ends in the phase it started in");
 
 } // namespace
 
@@ -60,8 +62,8 @@ struct gol_engine {
     bool local = false;
     golb200::LocalPlan lplan{};
     golb200::LocalState lst{};
-    int lparity = 0;                       // pass parity of the change flags
-    cudaGraphExec_t lchunk[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};   // [cur][lparity]
+    int lphase = 0;                        // pass number mod kLocalPhases
+    cudaGraphExec_t lchunk[2][golb200::kLocalPhases] = {};   // [cur][lphase]
 
     std::string err;
 
@@ -135,13 +137,9 @@ int alloc_local(gol_engine* e) {
         }
     }
     // First pass of a round: every tile counts as changed.
-    const size_t cb = golb200::local_change_bytes(e->lplan);
-    ce = cudaMemsetAsync(s.changed[1], 0xff, cb, e->stream);
-    if (ce == cudaSuccess) ce = cudaMemsetAsync(s.changed[0], 0, cb, e->stream);
-    if (ce == cudaSuccess) ce = cudaMemsetAsync(s.pass_no, 0, sizeof(uint32_t), e->stream);
-    if (ce == cudaSuccess) ce = cudaMemsetAsync(s.count, 0, golb200::kLocalCountWords * sizeof(int), e->stream);
+    e->lphase = 0;
+    ce = golb200::reset_local(e->lplan, s, e->lphase, true, e->stream);
     if (ce != cudaSuccess) return e->cuda_fail(ce, "change-tracking reset");
-    e->lparity = 0;
     return GOL_OK;
 }
 
@@ -197,14 +195,14 @@ int launch_pass(gol_engine* e, int k, cudaStream_t s, int from) {
     return GOL_OK;
 }
 
-int launch_local(gol_engine* e, cudaStream_t s, int from, int parity) {
+int launch_local(gol_engine* e, cudaStream_t s, int from, int phase) {
     cudaError_t ce = golb200::launch_local_pass(e->d[from], e->d[from ^ 1], e->W, e->Y, e->k,
-                                                e->lplan, e->lst, parity, s);
+                                                e->lplan, e->lst, phase, s);
     if (ce != cudaSuccess) return e->cuda_fail(ce, "change-tracking pass launch");
     return GOL_OK;
 }
 
-int build_local_graph(gol_engine* e, int cur, int parity) {
+int build_local_graph(gol_engine* e, int cur, int phase) {
     if (!e->capture_stream) {
         cudaError_t ce = cudaStreamCreateWithFlags(&e->capture_stream, cudaStreamNonBlocking);
         if (ce != cudaSuccess) return e->cuda_fail(ce, "capture stream");
@@ -212,10 +210,10 @@ int build_local_graph(gol_engine* e, int cur, int parity) {
     cudaError_t ce = cudaStreamBeginCapture(e->capture_stream, cudaStreamCaptureModeThreadLocal);
     if (ce != cudaSuccess) return e->cuda_fail(ce, "begin capture");
     int rc = GOL_OK;
-    for (int i = 0; i < kGraphPasses && rc == GOL_OK; ++i) {
-        rc = launch_local(e, e->capture_stream, cur, parity);
+    for (int i = 0; i < kLocalGraphPasses && rc == GOL_OK; ++i) {
+        rc = launch_local(e, e->capture_stream, cur, phase);
         cur ^= 1;
-        parity ^= 1;
+        phase = (phase + 1) % golb200::kLocalPhases;
     }
     cudaGraph_t graph = nullptr;
     ce = cudaStreamEndCapture(e->capture_stream, &graph);
@@ -224,7 +222,7 @@ int build_local_graph(gol_engine* e, int cur, int parity) {
         return rc;
     }
     if (ce != cudaSuccess) return e->cuda_fail(ce, "end capture");
-    ce = cudaGraphInstantiate(&e->lchunk[cur][parity], graph, 0);
+    ce = cudaGraphInstantiate(&e->lchunk[cur][phase], graph, 0);
     cudaGraphDestroy(graph);
     if (ce != cudaSuccess) return e->cuda_fail(ce, "graph instantiate");
     return GOL_OK;
@@ -504,20 +502,20 @@ int gol_run(gol_engine* e, uint64_t n) {
     int rc;
     if (e->local) {
         if (budget == 0) {
-            while (passes >= (uint64_t)kGraphPasses) {
-                auto& g = e->lchunk[e->cur][e->lparity];
-                if (!g && (rc = build_local_graph(e, e->cur, e->lparity))) return rc;
+            while (passes >= (uint64_t)kLocalGraphPasses) {
+                auto& g = e->lchunk[e->cur][e->lphase];
+                if (!g && (rc = build_local_graph(e, e->cur, e->lphase))) return rc;
                 cudaError_t ce = cudaGraphLaunch(g, e->stream);
                 if (ce != cudaSuccess) return e->cuda_fail(ce, "graph launch");
-                passes -= kGraphPasses;          // even: cur and lparity come back
-                e->performed += (uint64_t)kGraphPasses * k;
+                passes -= kLocalGraphPasses;     // cur and lphase come back
+                e->performed += (uint64_t)kLocalGraphPasses * k;
             }
         }
         for (; passes > 0; --passes) {
             if (time_is_up()) return GOL_OK;
-            if ((rc = launch_local(e, e->stream, e->cur, e->lparity))) return rc;
+            if ((rc = launch_local(e, e->stream, e->cur, e->lphase))) return rc;
             e->cur ^= 1;
-            e->lparity ^= 1;
+            e->lphase = (e->lphase + 1) % golb200::kLocalPhases;
             e->performed += k;
         }
         if (rem > 0) {
@@ -527,8 +525,7 @@ int gol_run(gol_engine* e, uint64_t n) {
             if ((rc = launch_pass(e, rem, e->stream, e->cur))) return rc;
             e->cur ^= 1;
             e->performed += rem;
-            cudaError_t ce = cudaMemsetAsync(e->lst.changed[e->lparity ^ 1], 0xff,
-                                             golb200::local_change_bytes(e->lplan), e->stream);
+            cudaError_t ce = golb200::reset_local(e->lplan, e->lst, e->lphase, false, e->stream);
             if (ce != cudaSuccess) return e->cuda_fail(ce, "change-flag reset");
         }
         return GOL_OK;

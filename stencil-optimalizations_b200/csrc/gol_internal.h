@@ -127,6 +127,7 @@ struct LocalPlan {
     int num_sms = 0;
     RowsPlan dense;    // the dense form of a pass (row bands over the whole grid)
     int dense_min = 0; // active tiles from which a pass runs dense (INT_MAX = never)
+    int block = 0;     // rows in registers of the one-kernel form (0: plan, dense and tile kernels)
 };
 
 // Word layouts (gol_layouts.cu): X_BITS x Y_BITS cells per word.
@@ -156,7 +157,8 @@ inline size_t local_list_ints(const LocalPlan& lp) {
 }
 
 struct LocalState {
-    uint32_t* changed[2] = {nullptr, nullptr};  // change bits per tile, by pass parity
+    uint32_t* changed[3] = {nullptr, nullptr, nullptr};   // change bits per tile, by pass (mod 3
+                                                // in the one-kernel form, else by parity)
     int* list = nullptr;                        // active tiles of the current pass
     int* count = nullptr;                       // kLocalCountWords plan words: tile counts
                                                 // by pass parity, CTA ticket, dense choice
@@ -170,12 +172,17 @@ struct LocalState {
 bool plan_local_tiles(int W, int Y, int k, int tile_rows, int wpl, int num_sms, int dense_pct,
                       LocalPlan* lp);
 
-// One change-tracking pass: plan (reads changed[parity ^ 1], clears
-// changed[parity]) then the tile kernel or, from dense_min active tiles, the
-// dense tracked kernel (either writes changed[parity]).
+// Pass `phase` (mod kLocalPhases) of a change-tracking run: it reads the
+// previous pass's change bits and writes its own, in one kernel, or as a plan
+// and then the tile kernel or, from dense_min active tiles, the dense tracked
+// kernel.
+constexpr int kLocalPhases = 6;   // the flag buffers and counters repeat by 3 and by 2
 cudaError_t launch_local_pass(const uint32_t* src, uint32_t* dst, int W, int Y, int k,
-                              const LocalPlan& lp, const LocalState& st, int parity,
+                              const LocalPlan& lp, const LocalState& st, int phase,
                               cudaStream_t stream);
+// Lets pass `phase` find every tile changed; counts: starts a run's counters.
+cudaError_t reset_local(const LocalPlan& lp, const LocalState& st, int phase, bool counts,
+                        cudaStream_t stream);
 
 // Batched uneven grids (one persistent launch over a work list).
 struct BatchGrid {

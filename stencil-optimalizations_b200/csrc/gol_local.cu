@@ -11,7 +11,9 @@
 // the unknown cells beyond it, whose errors move one cell per generation)
 // times a band of rows, so
 // the skip rule needs tiles at least K cells high and wide (a pass reads K
-// cells around each cell). Per pass:
+// cells around each cell). Tiles of one word and of up to 64 - 2K rows (the
+// default) run in one kernel per pass (local_pass_kernel below); wider and
+// taller ones per pass in three:
 //   plan   one thread per 32 tiles of a tile row dilates the previous
 //          pass's change bits over the 3x3 neighbourhood, active tiles are
 //          appended to a list as runs (warp scan + one atomic per warp), this pass's
@@ -40,6 +42,7 @@
 #include <climits>
 
 #include "gol_internal.h"
+#include "gol_rows_block.cuh"
 #include "gol_rows_temporal.cuh"
 
 #ifndef GOL_LOCAL_CARVEOUT
@@ -76,6 +79,8 @@ __host__ __device__ inline int change_words(int tiles_x) { return (tiles_x + 31)
 // length by pass parity.
 enum PlanCounts { kTiles0 = 0, kTicket = 2, kDenseHint = 3, kDense0 = 4, kLanes0 = 6 };
 static_assert(kLanes0 + 2 <= kLocalCountWords, "plan words");
+// The one-kernel form's: its tally (two words), the dense hints by parity.
+constexpr int kHint0 = 2;
 
 // The lane list: a pass's active tiles in runs of horizontally adjacent
 // tiles of one tile row, each run with a halo lane before and after it. An
@@ -326,6 +331,228 @@ rows_tracked_kernel(RowsLaunch a, TileTrack tt, const int* __restrict__ dense, i
         band_tile<WPL, K, 2>(a, u % nbands, u / nbands, smem, tt);
 }
 
+// One-kernel form of a pass, for tiles of one word by a height that fits in
+// registers (the default tiles among them): every warp dilates the change
+// bits of a few flag words of its own, its CTA lists their active tiles in
+// shared memory as runs (the same runs and halo lanes as above) and its warps
+// compute them window by window, a tile's rows + 2K rows in each lane's
+// registers (gol_rows_block.cuh). A CTA owns its flag words, so it writes them
+// whole: no list in memory, no second kernel that waits for it, no atomics on
+// the flags. A pass is bound by its latency (launch, flag words, rows,
+// generations, in a chain): 5.0 us with 760 of 1.4 M tiles active, 7.6 us with
+// 14000, 13.8 us with 54000 (16384^2, k = 6), where the three kernels above
+// took 13.3, 16.1 and 23.4 us. Tiles of a whole run need no dead words at the
+// run's ends: a halo lane takes the errors from beyond it.
+//
+// Flag words go to warps in chunks of eight (one 32-byte sector), chunk c to
+// warp c mod all warps: activity clusters, and a cluster's tile rows then fall
+// to different CTAs.
+//
+// A pass whose predecessor counted at least dense_min active tiles runs dense:
+// the same warps walk blocks of rows by 30 columns of the whole grid instead
+// and OR the change bits of the tiles that differ into flag words that the
+// pass before cleared (three flag buffers in turn: read, written, cleared). A
+// round starts with that hint set, as every tile is active then. (Every tile
+// active, 16384^2, k = 6: 75 us a pass against 78 for rows_tracked_kernel.)
+struct LocalPass {
+    const uint32_t* src;
+    uint32_t* dst;
+    int W, Y;
+    int rows, K;               // tile height, generations
+    int cw, nwords;            // flag words per tile row, in all
+    const uint32_t* prev;      // the previous pass's change bits
+    uint32_t* cur;             // this pass's (zero on entry)
+    uint32_t* clear;           // the next pass's, zeroed here
+    int dense_rows, dense_blocks, dense_wins;   // the dense form's blocks and warps' windows
+    int dense_min;
+    int ntiles;
+    const int* hint;           // nonzero: this pass runs dense
+    int* next_hint;
+    unsigned long long* tally; // active tiles << 32 | warps done
+    uint32_t* census;
+    uint32_t census_cap;
+    uint32_t* pass_no;
+};
+
+constexpr int kLocalChunks = 4;     // chunks of eight flag words per warp, at most (a lane per word)
+constexpr int kLocalWarps = 4;      // warps per CTA, which share one list
+// Warps per SM of the one wave a pass runs: on the sparse workload's passes of
+// 54000, 14000 and 760 active tiles 12 / 16 / 20 ran at 14.9 / 13.8 / 13.6,
+// 7.8 / 7.6 / 8.0 and 4.9 / 5.0 / 5.5 us, its dense passes at 82 / 75 / 66 us.
+constexpr int kLocalWaveWarps = 16;
+constexpr int kDenseR = 64;         // rows in registers of the dense form (a bit per row below)
+
+template <int R>
+__global__ void __launch_bounds__(32 * kLocalWarps, 5) local_pass_kernel(LocalPass a) {
+    constexpr int kWords = 32 * kLocalWarps;
+    __shared__ uint16_t list[kWords * 48];   // owner << 7 | bit << 2 | role
+    __shared__ uint32_t flags[kWords];
+    __shared__ int word_y[kWords], word_x[kWords];
+    __shared__ int warp_lanes[kLocalWarps], warp_tiles[kLocalWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int gwarp = blockIdx.x * kLocalWarps + warp, nwarps = gridDim.x * kLocalWarps;
+    // This lane's flag word.
+    const long long t = ((long long)(lane >> 3) * nwarps + gwarp) * 8 + (lane & 7);
+    const bool mine = (lane >> 3) < kLocalChunks && t < a.nwords;
+    const int ty = mine ? (int)t / a.cw : 0, wx = mine ? (int)t - ty * a.cw : 0;
+    const bool above = ty > 0, below = ty + 1 < a.nwords / a.cw;
+    const bool left = wx > 0, right = wx + 1 < a.cw;
+    flags[threadIdx.x] = 0u;
+    word_y[threadIdx.x] = ty;
+    word_x[threadIdx.x] = wx;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const bool dense = __ldcg(a.hint) != 0;
+    uint32_t act = 0u;
+    if (mine) {
+#pragma unroll
+        for (int dy = -1; dy <= 1; ++dy) {
+            const bool in = dy < 0 ? above : dy == 0 || below;
+            const uint32_t* row = a.prev + t + dy * a.cw;
+            const uint32_t v = in ? row[0] : 0u;
+            const uint32_t l = in && left ? row[-1] : 0u;
+            const uint32_t r = in && right ? row[1] : 0u;
+            act |= v | (v << 1) | (l >> 31) | (v >> 1) | (r << 31);
+        }
+        const int valid = a.W - 32 * wx;   // tiles (words) in this flag word
+        if (valid < 32) act &= (1u << valid) - 1u;
+        a.clear[t] = 0u;
+    }
+    // Runs continue from lane to lane within a chunk and a tile row.
+    const uint32_t prev_act = __shfl_up_sync(0xffffffffu, act, 1);
+    const uint32_t next_act = __shfl_down_sync(0xffffffffu, act, 1);
+    const bool cin = (lane & 7) > 0 && wx > 0 && (prev_act >> 31);
+    const bool cout = (lane & 7) < 7 && wx + 1 < a.cw && (next_act & 1u);
+    const uint32_t starts = act & ~((act << 1) | (cin ? 1u : 0u));
+    const uint32_t ends = act & ~((act >> 1) | (cout ? 0x80000000u : 0u));
+    const int n = __popc(act);
+    const int packed = ((n + __popc(starts) + __popc(ends)) << 16) | n;
+    int incl = packed;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane == 31) {
+        warp_lanes[warp] = incl >> 16;
+        warp_tiles[warp] = incl & 0xffff;
+    }
+    __syncthreads();
+    int nl = 0, at = (incl - packed) >> 16, tiles = 0;
+#pragma unroll
+    for (int v = 0; v < kLocalWarps; ++v) {
+        if (v < warp) at += warp_lanes[v];
+        nl += warp_lanes[v];
+        tiles += warp_tiles[v];
+    }
+    // The last CTA records the pass (tiles computed: all of them when dense).
+    if (threadIdx.x == 0) {
+        const unsigned long long add = ((unsigned long long)tiles << 32) | 1ull;
+        const unsigned long long sum = atomicAdd(a.tally, add) + add;
+        if ((uint32_t)sum == gridDim.x) {
+            const int active = (int)(sum >> 32);
+            *a.next_hint = active >= a.dense_min ? 1 : 0;
+            const uint32_t p = __ldcg(a.pass_no);
+            if (p < a.census_cap) a.census[p] = dense ? (uint32_t)a.ntiles : (uint32_t)active;
+            *a.pass_no = p + 1;
+            *a.tally = 0ull;
+        }
+    }
+    if (!dense) {
+        for (uint32_t m = act; m; m &= m - 1u) {
+            const int b = __ffs((int)m) - 1;
+            const int e = (int)threadIdx.x << 7 | b << 2;
+            if ((starts >> b) & 1u) list[at++] = (uint16_t)(e | kRoleLeft);
+            list[at++] = (uint16_t)(e | kRoleTile);
+            if ((ends >> b) & 1u) list[at++] = (uint16_t)(e | kRoleRight);
+        }
+        __syncthreads();
+        for (int w0 = warp * kWindowOwn; w0 < nl; w0 += kLocalWarps * kWindowOwn) {
+            // Lanes past either end of the list repeat its first or last
+            // entry, and store nothing.
+            const int g = w0 - 1 + lane;
+            const int d = list[min(max(g, 0), nl - 1)];
+            const int role = d & 3, bit = (d >> 2) & 31, owner = d >> 7;
+            const int tile_y = word_y[owner];
+            const int col = 32 * word_x[owner] + bit +
+                            (role == kRoleLeft ? -1 : role == kRoleRight ? 1 : 0);
+            const int y0 = tile_y * a.rows - a.K;
+            const bool ok = col >= 0 && col < a.W;
+            const bool inside = __all_sync(0xffffffffu, ok && y0 >= 0 && y0 + R <= a.Y);
+            uint32_t w[R];
+            block_load<R>(w, a.src + (long long)y0 * a.W + col, a.W, inside, ok, y0, a.Y);
+            block_generations<R>(w, a.rows, a.K, inside, ok, y0, a.Y);
+            const bool own = role == kRoleTile && lane >= 1 && lane <= kWindowOwn && g < nl;
+            const int rows = min(a.rows, a.Y - tile_y * a.rows);
+            const uint32_t* old = a.src + (long long)tile_y * a.rows * a.W + col;
+            uint32_t* out = a.dst + (long long)tile_y * a.rows * a.W + col;
+            uint32_t diff = 0u;
+            if (own) {
+#pragma unroll
+                for (int r = 0; r < R - 2; ++r, old += a.W, out += a.W) {
+                    if (r < rows) {
+                        diff |= w[r] ^ __ldg(old);
+                        *out = w[r];
+                    }
+                }
+                if (diff) atomicOr(flags + owner, 1u << bit);
+            }
+        }
+        __syncthreads();
+        if (mine) a.cur[t] = flags[threadIdx.x];
+    } else {
+        const long long line = a.W + 1;
+        for (int win = gwarp; win < a.dense_wins; win += nwarps) {
+            const long long idx = (long long)win * kBlockOwn - 1 + lane;
+            const int block = idx < 0 ? 0 : (int)(idx / line);
+            const int col = (int)(idx - block * line);
+            const bool ok = idx >= 0 && block < a.dense_blocks && col < a.W;
+            const bool own = ok && lane >= 1 && lane <= kBlockOwn;
+            const int ys = block * a.dense_rows, y0 = ys - a.K;
+            const bool inside = __all_sync(0xffffffffu, ok && y0 >= 0 && y0 + kDenseR <= a.Y);
+            uint32_t w[kDenseR];
+            block_load<kDenseR>(w, a.src + (long long)y0 * a.W + col, a.W, inside, ok, y0, a.Y);
+            block_generations<kDenseR>(w, a.dense_rows, a.K, inside, ok, y0, a.Y);
+            // Lanes of one flag word close each tile row together. (The loop
+            // below is uniform: it covers the block's full height, rows past
+            // the grid differ in nothing.)
+            long long word = own ? (long long)(ys / a.rows) * a.cw + (col >> 5) : -1;
+            const unsigned group = __match_any_sync(0xffffffffu, word);
+            const bool leader = own && (int)(__ffs((int)group) - 1) == lane;
+            const uint32_t* old = a.src + (long long)ys * a.W + col;
+            uint32_t* out = a.dst + (long long)ys * a.W + col;
+            const int rows = own ? min(a.dense_rows, a.Y - ys) : 0;
+            unsigned long long changed = 0ull;   // bit r: row r of the block differs
+#pragma unroll
+            for (int r = 0; r < kDenseR - 2; ++r, old += a.W, out += a.W) {
+                if (r < rows) {
+                    if (w[r] != __ldg(old)) changed |= 1ull << r;
+                    *out = w[r];
+                }
+            }
+            for (int r = 0; r < a.dense_rows; r += a.rows, word += a.cw) {
+                const bool diff = (changed >> r & ((1ull << a.rows) - 1ull)) != 0ull;
+                const uint32_t bits = __reduce_or_sync(group, diff ? 1u << (col & 31) : 0u);
+                if (leader && bits) atomicOr(a.cur + word, bits);
+            }
+        }
+    }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <int R>
+cudaError_t launch_local_one(const LocalPass& a, int warps, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((warps + kLocalWarps - 1) / kLocalWarps));
+    cfg.blockDim = dim3(32 * kLocalWarps);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, local_pass_kernel<R>, a);
+}
+
 // Lane width of the dense tracked pass for depth k: the widest whose
 // register rings fit (one kernel per depth).
 constexpr int tracked_wpl(int k) { return k <= kMaxKForWpl(4) ? 4 : (k <= kMaxKForWpl(2) ? 2 : 1); }
@@ -436,6 +663,8 @@ bool plan_local_tiles(int W, int Y, int k, int tile_rows, int wpl, int num_sms, 
     const long long windows = (lanes + kWindowOwn - 1) / kWindowOwn;
     lp->ctas = (int)std::max(1LL, (std::min<long long>(windows, num_sms * 24LL) + kTileWarps - 1) / kTileWarps);
     lp->num_sms = num_sms;
+    // One kernel per pass where a tile's rows fit in a lane's registers.
+    lp->block = wpl != 1 ? 0 : band + 2 * k <= 20 ? 20 : band + 2 * k <= 32 ? 32 : band + 2 * k <= 64 ? 64 : 0;
     // The dense form: the row-band plan at the kernel's lane width. Its
     // lanes start at multiples of that width and tiles are 1, 2 or 4 words
     // wide (or the whole row), so no lane straddles two change words.
@@ -443,16 +672,85 @@ bool plan_local_tiles(int W, int Y, int k, int tile_rows, int wpl, int num_sms, 
     const long long ntiles = (long long)lp->tiles_x * lp->tiles_y;
     if (dense_pct == 0) dense_pct = GOL_LOCAL_DENSE_PCT;
     lp->dense_min = INT_MAX;
+    if (lp->block) {
+        if (dense_pct <= 100) lp->dense_min = (int)std::max(1LL, (ntiles * dense_pct + 99) / 100);
+        return true;
+    }
     if (dense_pct <= 100 && plan_rows(W, Y, k, 0, tracked_wpl(k), num_sms, &lp->dense, true))
         lp->dense_min = (int)std::max(1LL, (ntiles * dense_pct + 99) / 100);
     return true;
 }
 
+cudaError_t reset_local(const LocalPlan& lp, const LocalState& st, int phase, bool counts,
+                        cudaStream_t stream) {
+    const size_t cb = local_change_bytes(lp);
+    const int prev = lp.block ? (phase + 2) % 3 : (phase & 1) ^ 1;
+    cudaError_t e = cudaMemsetAsync(st.changed[prev], 0xff, cb, stream);
+    if (counts) {
+        if (e == cudaSuccess) e = cudaMemsetAsync(st.changed[lp.block ? phase % 3 : phase & 1], 0, cb, stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(st.pass_no, 0, sizeof(uint32_t), stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(st.count, 0, kLocalCountWords * sizeof(int), stream);
+    }
+    // Every tile counts as active: dense, unless dense passes are off.
+    if (e == cudaSuccess && lp.block && lp.dense_min <= lp.tiles_x * lp.tiles_y)
+        e = cudaMemsetAsync(st.count + kHint0 + (phase & 1), 1, sizeof(int), stream);
+    return e;
+}
+
 cudaError_t launch_local_pass(const uint32_t* src, uint32_t* dst, int W, int Y, int k,
-                              const LocalPlan& lp, const LocalState& st, int parity,
+                              const LocalPlan& lp, const LocalState& st, int phase,
                               cudaStream_t stream) {
     const RowsPlan& p = lp.rows;
     const int nwords = change_words(lp.tiles_x) * lp.tiles_y;
+    const int parity = phase & 1;
+    if (lp.block) {
+        LocalPass a{};
+        a.src = src;
+        a.dst = dst;
+        a.W = W;
+        a.Y = Y;
+        a.rows = p.band;
+        a.K = k;
+        a.cw = change_words(lp.tiles_x);
+        a.nwords = nwords;
+        a.prev = st.changed[(phase + 2) % 3];
+        a.cur = st.changed[phase % 3];
+        a.clear = st.changed[(phase + 1) % 3];
+        a.dense_min = lp.dense_min;
+        a.ntiles = lp.tiles_x * lp.tiles_y;
+        a.hint = st.count + kHint0 + parity;
+        a.next_hint = st.count + kHint0 + (parity ^ 1);
+        a.tally = reinterpret_cast<unsigned long long*>(st.count);
+        a.census = st.census;
+        a.census_cap = st.census_cap;
+        a.pass_no = st.pass_no;
+        // One wave of warps where that covers the flag words (at most
+        // kLocalChunks chunks each), fewer on small grids.
+        const int chunks = (nwords + 7) / 8;
+        const int warps = std::max(std::min(chunks, kLocalWaveWarps * lp.num_sms),
+                                   (chunks + kLocalChunks - 1) / kLocalChunks);
+        // The dense form's block height: whole tile rows, and the fewest
+        // row-generations for the warp with the most blocks (a block costs
+        // about 25 row-generations beside its own).
+        double best = 0;
+        for (int rows = p.band; rows <= kDenseR - 2 * k; rows += p.band) {
+            const long long blocks = ((long long)Y + rows - 1) / rows;
+            const long long wins = (blocks * (W + 1) + kBlockOwn - 1) / kBlockOwn;
+            const double cost = (double)((wins + warps - 1) / warps) * (k * (rows + k + 1.5) + 25);
+            if (wins > INT_MAX || (best > 0 && cost >= best)) continue;
+            best = cost;
+            a.dense_rows = rows;
+            a.dense_blocks = (int)blocks;
+            a.dense_wins = (int)wins;
+        }
+        if (best == 0) return cudaErrorInvalidConfiguration;
+        switch (lp.block) {
+            case 20: return launch_local_one<20>(a, warps, stream);
+            case 32: return launch_local_one<32>(a, warps, stream);
+            case 64: return launch_local_one<64>(a, warps, stream);
+            default: return cudaErrorInvalidValue;
+        }
+    }
     static const cudaError_t plan_attr = set_carveout(plan_tiles_kernel);
     if (plan_attr != cudaSuccess) return plan_attr;
     plan_tiles_kernel<<<(nwords + kPlanThreads - 1) / kPlanThreads, kPlanThreads, 0, stream>>>(

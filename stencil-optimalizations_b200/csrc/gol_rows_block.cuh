@@ -63,30 +63,30 @@ __device__ __forceinline__ void block_hsum(uint32_t c, uint32_t& h0, uint32_t& h
     hsum(lw, c, rw, h0, h1);
 }
 
+// Rows y0 .. y0 + R - 1 of one column into registers (p points at row y0 of
+// it; it is dereferenced inside the grid only). inside: every row and column
+// of the warp lies in the grid; ok: this lane's column does.
 template <int R>
-__global__ void __launch_bounds__(32, block_min_ctas<R>()) rows_block_kernel(BlockLaunch a) {
-    static_assert(R % 4 == 0, "rows are taken two at a time, the exit tested every four");
-    const int lane = threadIdx.x;
-    const long long line = a.W + 1;
-    const long long idx = (long long)blockIdx.x * kBlockOwn - 1 + lane;
-    const int block = idx < 0 ? 0 : (int)(idx / line);
-    const int col = (int)(idx - block * line);   // -1: before the first column, W: a dead column
-    const bool ok = idx >= 0 && block < a.nblocks && col < a.W;
-    const int y0 = block * a.B - a.K;            // row of w[0]
-    const bool inside = __all_sync(0xffffffffu, ok && y0 >= 0 && y0 + R <= a.Y);
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    uint32_t w[R];
-    const uint32_t* p = a.src + (long long)y0 * a.pitch + col;   // dereferenced inside the grid only
+__device__ __forceinline__ void block_load(uint32_t (&w)[R], const uint32_t* p, int pitch,
+                                           bool inside, bool ok, int y0, int Y) {
     if (inside) {
 #pragma unroll
-        for (int r = 0; r < R; ++r, p += a.pitch) w[r] = __ldg(p);
+        for (int r = 0; r < R; ++r, p += pitch) w[r] = __ldg(p);
     } else {
 #pragma unroll
-        for (int r = 0; r < R; ++r, p += a.pitch)
-            w[r] = ok && (unsigned)(y0 + r) < (unsigned)a.Y ? __ldg(p) : 0u;
+        for (int r = 0; r < R; ++r, p += pitch)
+            w[r] = ok && (unsigned)(y0 + r) < (unsigned)Y ? __ldg(p) : 0u;
     }
-    for (int g = 1; g <= a.K; ++g) {
-        const int n = a.B + 2 * (a.K - g);   // rows that count after this generation
+}
+
+// K generations of the block in w (rows y0 ..): afterwards w[0 .. B-1] are
+// rows y0 + K .. y0 + K + B - 1 (B + 2K <= R).
+template <int R>
+__device__ __forceinline__ void block_generations(uint32_t (&w)[R], int B, int K, bool inside,
+                                                  bool ok, int y0, int Y) {
+    static_assert(R % 4 == 0, "rows are taken two at a time, the exit tested every four");
+    for (int g = 1; g <= K; ++g) {
+        const int n = B + 2 * (K - g);   // rows that count after this generation
         uint32_t a0, a1, b0, b1;
         block_hsum(w[0], a0, a1);
         block_hsum(w[1], b0, b1);
@@ -109,9 +109,25 @@ __global__ void __launch_bounds__(32, block_min_ctas<R>()) rows_block_kernel(Blo
         if (!inside) {   // columns and rows outside the grid stay dead
 #pragma unroll
             for (int r = 0; r < R; ++r)
-                w[r] = ok && (unsigned)(y0 + g + r) < (unsigned)a.Y ? w[r] : 0u;
+                w[r] = ok && (unsigned)(y0 + g + r) < (unsigned)Y ? w[r] : 0u;
         }
     }
+}
+
+template <int R>
+__global__ void __launch_bounds__(32, block_min_ctas<R>()) rows_block_kernel(BlockLaunch a) {
+    const int lane = threadIdx.x;
+    const long long line = a.W + 1;
+    const long long idx = (long long)blockIdx.x * kBlockOwn - 1 + lane;
+    const int block = idx < 0 ? 0 : (int)(idx / line);
+    const int col = (int)(idx - block * line);   // -1: before the first column, W: a dead column
+    const bool ok = idx >= 0 && block < a.nblocks && col < a.W;
+    const int y0 = block * a.B - a.K;            // row of w[0]
+    const bool inside = __all_sync(0xffffffffu, ok && y0 >= 0 && y0 + R <= a.Y);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    uint32_t w[R];
+    block_load<R>(w, a.src + (long long)y0 * a.pitch + col, a.pitch, inside, ok, y0, a.Y);
+    block_generations<R>(w, a.B, a.K, inside, ok, y0, a.Y);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (ok && lane >= 1 && lane <= kBlockOwn) {
         const int ys = block * a.B;
