@@ -38,6 +38,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <mutex>
 #include <new>
@@ -359,6 +360,29 @@ batch_kernel(const BatchGrid* __restrict__ grids, const BatchItem* __restrict__ 
     }
 }
 
+// Many grids: persistent CTAs (all resident: a cooperative launch) take
+// bands in ticket order and run each to its last generation. The bands of a
+// grid have consecutive tickets, so a band's neighbours are always taken by
+// CTAs that are running or will be as soon as one frees up: a grid has at
+// most as many bands as there are CTAs, and bands of earlier grids never
+// wait on later tickets.
+__global__ void __launch_bounds__(kResidentMaxThreads, 1)
+batch_resident_kernel(const ResidentBand* __restrict__ jobs, int njobs, int* ticket, int* status,
+                      long long spin_limit) {
+    extern __shared__ __align__(16) uint32_t smem[];
+    __shared__ int stop;
+    __shared__ int job;
+    for (;;) {
+        if (threadIdx.x == 0) job = atomicAdd(ticket, 1);
+        __syncthreads();
+        const int t = job;
+        if (t >= njobs) return;
+        const ResidentBand j = jobs[t];
+        if (!resident_band<0>(j, smem, &stop, status, spin_limit)) return;
+        __syncthreads();   // shared memory and `job` are reused by the next band
+    }
+}
+
 } // namespace
 
 // ---------------------------------------------------------------------------
@@ -576,28 +600,11 @@ namespace golb200 {
 #ifndef GOL_RBATCH_K
 #define GOL_RBATCH_K 8
 #endif
-#ifndef GOL_RBATCH_ROWS_PER_GROUP
-#define GOL_RBATCH_ROWS_PER_GROUP 8
-#endif
-#ifndef GOL_RBATCH_BANDS_PER_CTA
-#define GOL_RBATCH_BANDS_PER_CTA 3
-#endif
 namespace {
-constexpr int kResidentBatchWpl = 2;        // words per lane of the resident batch kernel
 constexpr int kResidentBatchThreads = 512;  // threads per CTA
 constexpr int kResidentBatchK = GOL_RBATCH_K;   // generations per epoch
-constexpr int kResidentBatchRowsPerGroup = GOL_RBATCH_ROWS_PER_GROUP;   // fewer rows per group and
-                                                                        // pass cost warm-up
-constexpr int kResidentBatchBandsPerCta = GOL_RBATCH_BANDS_PER_CTA;     // about this many bands per
-                                                                        // CTA (balance)
 } // namespace
 
-// Per grid: lanes of two words across its row and row groups over the CTA's
-// threads; as many bands as the shared memory needs, more for grids whose
-// work would otherwise make one band a long job (about
-// kResidentBatchBandsPerCta bands per CTA over the batch), fewer where a
-// band would give a row group under kResidentBatchRowsPerGroup rows; every
-// band of a grid at least K rows, at most one band per SM.
 namespace {
 // Per device: the opt-in shared memory per CTA, with the kernel's dynamic
 // shared memory limit raised to it (once), and the resident CTAs per SM by
@@ -616,7 +623,7 @@ const char* resident_device(int device, size_t smem, int* smem_optin, int* per_s
     if (!d.smem_optin) {
         int v = 0;
         if (cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess ||
-            cudaFuncSetAttribute(batch_resident_kernel<kResidentBatchWpl>,
+            cudaFuncSetAttribute(batch_resident_kernel,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, v - 1024) != cudaSuccess)
             return "device attribute";
         d.smem_optin = v;
@@ -628,7 +635,7 @@ const char* resident_device(int device, size_t smem, int* smem_optin, int* per_s
         if (it == d.per_sm.end()) {
             int n = 0;
             if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                    &n, batch_resident_kernel<kResidentBatchWpl>, kResidentBatchThreads,
+                    &n, batch_resident_kernel, kResidentBatchThreads,
                     std::min<size_t>(key, (size_t)d.smem_optin - 1024)) != cudaSuccess)
                 return "resident batch occupancy";
             it = d.per_sm.emplace(key, n).first;
@@ -639,41 +646,136 @@ const char* resident_device(int device, size_t smem, int* smem_optin, int* per_s
 }
 } // namespace
 
+// The grids a resident batch takes: rows of up to 1024 words, and as many
+// bands as needed where a band's two buffers of (rows + 2K) rows fit with
+// rows of W words padded to even and eight more (the kernel's are no longer).
+namespace {
+constexpr int kResidentBatchMaxW = 1024;
+long long resident_batch_rows(size_t avail, int W, int K) {
+    return (long long)(avail / (2ull * ((W + 1) / 2 * 2 + 8) * sizeof(uint32_t))) - 2 * K;
+}
+} // namespace
+
+namespace {
+// Estimated SM cycles per generation of a band of `rows` rows of `lanes` lanes
+// (four words each): row groups of two rows or more over the CTA's threads, a
+// part per lane and row (34 operations, and 10 per group for its first two
+// rows' sums, at 64 lanes a cycle, and what is lost beside: a quarter, two
+// fifths where row groups share a warp and its banks), and a fixed part for
+// the barriers and, unless the grid is one band, the exchange. Fitted to
+// batches of equal grids of 256^2 .. 4096^2 to about 15 %.
+int band_groups(int lanes, int rows, int K) {
+    return std::max(1, std::min(kResidentBatchThreads / lanes, (rows + K + 1) / 2));
+}
+double band_cycles(int lanes, double rows, bool alone) {
+    const double r = rows + (alone ? 0 : kResidentBatchK - 1);
+    return (alone ? 1000 : 1300) +
+           (lanes % 32 ? 1.4 : 1.25) * lanes / 64 *
+               (34 * r + 10 * band_groups(lanes, (int)rows, kResidentBatchK));
+}
+} // namespace
+
+// Per grid: lanes of four words across its row, row groups over the CTA's
+// threads, and bands. A batch takes about max(longest band, all bands / SMs),
+// and cutting a grid finer shortens its bands but adds halo rows and
+// exchanges, so the planner searches the longest band's time T: every grid
+// takes the fewest bands whose time stays within T (never fewer than its
+// shared memory needs, every band at least K rows, at most one band per SM),
+// and the T whose schedule ends first wins.
 const char* plan_resident_batch(const ResidentGrid* g, size_t n, int num_sms, int device,
                                 ResidentBatchPlan* p) {
     int smem_optin = 0;
     if (const char* why = resident_device(device, 0, &smem_optin, nullptr)) return why;
     const size_t avail = (size_t)smem_optin - 1024;
-    double total = 0;
-    for (size_t i = 0; i < n; ++i) total += (double)g[i].W * g[i].Y * g[i].gens;
+    struct Cut {
+        int lanes, K, lo, hi;   // bands: at least, at most
+        size_t row_bytes;
+    };
+    std::vector<Cut> cuts(n);
+    double longest = 0;
+    for (size_t i = 0; i < n; ++i) {
+        const ResidentGrid& e = g[i];
+        if (e.W > kResidentBatchMaxW) return "a grid is too wide for the resident batch";
+        Cut& c = cuts[i];
+        c.lanes = (e.W + 3) / 4;
+        c.K = (int)std::min<long long>(e.gens, kResidentBatchK);
+        c.row_bytes = 2ull * resident_stride(c.lanes) * 4;
+        const long long fit = (long long)(avail / c.row_bytes) - 2 * c.K;   // band rows that fit
+        const long long accepted = resident_batch_rows(avail, e.W, c.K);
+        if (fit < 1 || accepted < 1) return "a grid's rows do not fit in shared memory";
+        c.hi = std::min(num_sms, std::max(1, e.Y / c.K));
+        if ((e.Y + accepted - 1) / accepted > c.hi)
+            return "a grid needs more bands than the GPU runs at once, or bands under K rows";
+        c.lo = (int)((e.Y + fit - 1) / fit);
+        longest = std::max(longest, (double)e.gens * band_cycles(c.lanes, (double)e.Y / c.lo, c.lo == 1));
+    }
+    auto band_time = [&](size_t i, int nb) {
+        return (double)g[i].gens * band_cycles(cuts[i].lanes, (double)g[i].Y / nb, nb == 1);
+    };
+    auto bands_within = [&](size_t i, double T) {   // the fewest bands that stay within T
+        const Cut& c = cuts[i];
+        if (band_time(i, c.lo) <= T) return c.lo;
+        int lo = c.lo, hi = c.hi;   // lo is over T; times fall from two bands on
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) / 2;
+            (band_time(i, mid) <= T ? hi : lo) = mid;
+        }
+        return band_time(i, hi) < band_time(i, c.lo) ? hi : c.lo;
+    };
+    // The batch's end with bands in ticket order: a grid's bands run together,
+    // so it starts when the last of its CTAs falls free. Bands take what they
+    // take, not what was estimated, and a schedule that fits by luck is not
+    // wanted: the mean of three runs with times up to a quarter longer.
+    struct Job {
+        double time;
+        int nb;
+        uint32_t id;
+    };
+    std::vector<Job> jobs(n);
+    std::vector<double> free_at;
+    auto ends_at = [&](double T) {
+        for (size_t i = 0; i < n; ++i) {
+            const int nb = bands_within(i, T);
+            jobs[i] = {band_time(i, nb), nb, (uint32_t)i};
+        }
+        std::sort(jobs.begin(), jobs.end(), [](const Job& x, const Job& y) { return x.time > y.time; });
+        double sum = 0;
+        for (uint32_t run = 1; run <= 3; ++run) {
+            free_at.assign(num_sms, 0.0);          // ascending
+            for (const auto& j : jobs) {
+                const uint32_t h = (j.id * 2654435761u + run * 0x9E3779B9u) >> 24;   // 0 .. 255
+                const double t = free_at[j.nb - 1] + j.time * (1.0 + h / 1024.0);
+                const auto at = std::upper_bound(free_at.begin() + j.nb, free_at.end(), t);
+                std::fill(std::move(free_at.begin() + j.nb, at, free_at.begin()), at, t);
+            }
+            sum += free_at.back();
+        }
+        return sum;
+    };
+    // T from the longest uncut band down, a sixth less each time, until the
+    // end has only grown for a while.
+    double best = -1, best_T = longest;
+    int worse = 0;
+    for (double T = longest; worse < 4 && T > longest / 100; T *= 5.0 / 6.0) {
+        // (a long band that starts late, behind misjudged ones, ends late)
+        const double end = ends_at(T) / 3 + 0.3 * T;
+        if (best < 0 || end < best) {
+            best = end;
+            best_T = T;
+            worse = 0;
+        } else {
+            ++worse;
+        }
+    }
     std::vector<std::pair<double, ResidentBatchPlan::Grid>> order;
     size_t smem = 0;
     for (size_t i = 0; i < n; ++i) {
-        const ResidentGrid& e = g[i];
-        const int lanes = (e.W + kResidentBatchWpl - 1) / kResidentBatchWpl;
-        if (lanes > kResidentBatchThreads) return "a grid is too wide for the resident batch";
-        const int groups = kResidentBatchThreads / lanes;
-        const int K = (int)std::min<long long>(e.gens, kResidentBatchK);
-        const size_t row_bytes = 2ull * resident_stride(lanes, kResidentBatchWpl) * 4;
-        const long long fit = (long long)(avail / row_bytes) - 2 * K;   // band rows that fit
-        if (fit < 1) return "a grid's rows do not fit in shared memory";
-        const int nb_min = (int)((e.Y + fit - 1) / fit);
-        const double work = (double)e.W * e.Y * e.gens;
-        const int nb_work = (int)std::ceil(work / std::max(1.0, total / ((double)num_sms *
-                                                                          kResidentBatchBandsPerCta)));
-        const int nb_rows = std::max(1, e.Y / std::max(K, kResidentBatchRowsPerGroup * groups));
-        int nb = std::max(nb_min, std::min(nb_work, nb_rows));
-        // at most one band per SM (every CTA may hold the largest shared
-        // memory), every band at least K rows
-        const int nb_cap = std::min(num_sms, std::max(1, e.Y / K));
-        if (nb > nb_cap) {
-            if (nb_min > nb_cap) return "a grid needs more bands than the GPU runs at once, or bands under K rows";
-            nb = nb_cap;
-        }
-        const int B = (e.Y + nb - 1) / nb;
-        smem = std::max(smem, (size_t)(B + 2 * K) * row_bytes);
-        ResidentBatchPlan::Grid pg{(int)i, nb, K, lanes, groups, (e.W + 3) / 4 * 4, 0, 0};
-        order.push_back({(double)e.W * B * e.gens, pg});
+        const Cut& c = cuts[i];
+        const int nb = bands_within(i, best_T);
+        const int B = (g[i].Y + nb - 1) / nb;
+        smem = std::max(smem, (size_t)(B + 2 * c.K) * c.row_bytes);
+        ResidentBatchPlan::Grid pg{(int)i, nb, c.K, c.lanes, band_groups(c.lanes, B, c.K), 0};
+        order.push_back({band_time(i, nb), pg});
     }
     int per_sm = 0;
     if (const char* why = resident_device(device, smem, &smem_optin, &per_sm)) return why;
@@ -683,13 +785,12 @@ const char* plan_resident_batch(const ResidentGrid* g, size_t n, int num_sms, in
                      [](const auto& a, const auto& c) { return a.first > c.first; });
     p->grids.clear();
     p->pub_words = 0;
-    p->ndone = 0;
+    p->nbands = 0;
     for (auto& o : order) {
         if (o.second.nb > ctas) return "a grid needs more bands than CTAs";
         o.second.pub_off = p->pub_words;
-        o.second.done_off = p->ndone;
-        p->pub_words += (size_t)o.second.nb * 4 * o.second.K * o.second.ppitch;
-        p->ndone += o.second.nb;
+        p->pub_words += (size_t)o.second.nb * 4 * o.second.K * 4 * o.second.lanes;
+        p->nbands += o.second.nb;
         p->grids.push_back(o.second);
     }
     p->smem = smem;
@@ -700,16 +801,14 @@ const char* plan_resident_batch(const ResidentGrid* g, size_t n, int num_sms, in
 bool resident_batch_fits(int W, int Y, int num_sms, int device) {
     int smem_optin = 0;
     if (W <= 0 || Y <= 0 || resident_device(device, 0, &smem_optin, nullptr)) return false;
-    const int lanes = (W + kResidentBatchWpl - 1) / kResidentBatchWpl;
-    if (lanes > kResidentBatchThreads) return false;
-    const size_t row_bytes = 2ull * resident_stride(lanes, kResidentBatchWpl) * 4;
-    const long long fit = (long long)(((size_t)smem_optin - 1024) / row_bytes) - 2 * kResidentBatchK;
+    if (W > kResidentBatchMaxW) return false;
+    const long long fit = resident_batch_rows((size_t)smem_optin - 1024, W, kResidentBatchK);
     if (fit < 1) return false;
     const long long nb_min = (Y + fit - 1) / fit;
     return nb_min <= std::min(num_sms, std::max(1, Y / kResidentBatchK));
 }
 
-void fill_resident_jobs(const ResidentBatchPlan& p, const ResidentGrid* g, uint32_t* pub, int* done,
+void fill_resident_jobs(const ResidentBatchPlan& p, const ResidentGrid* g, unsigned long long* pub,
                         ResidentBand* jobs) {
     int t = 0;
     for (const auto& pg : p.grids) {
@@ -719,9 +818,7 @@ void fill_resident_jobs(const ResidentBatchPlan& p, const ResidentGrid* g, uint3
             j.src = e.src;
             j.dst = e.dst;
             j.pub = pub + pg.pub_off;
-            j.done = done + pg.done_off;
             j.pitch = e.pitch;
-            j.ppitch = pg.ppitch;
             j.W = e.W;
             j.Y = e.Y;
             j.K = pg.K;
@@ -739,7 +836,7 @@ cudaError_t launch_batch_resident(const ResidentBand* jobs, int njobs, int* tick
     // (the kernel's dynamic shared memory limit was raised when p was planned)
     long long spin = 1ll << 24;
     void* args[] = {&jobs, &njobs, &ticket, &status, &spin};
-    return cudaLaunchCooperativeKernel((const void*)batch_resident_kernel<kResidentBatchWpl>,
+    return cudaLaunchCooperativeKernel((const void*)batch_resident_kernel,
                                        dim3(p.ctas), dim3(kResidentBatchThreads), args, p.smem, stream);
 }
 
@@ -796,9 +893,8 @@ struct gol_batch {
     // exchange slots and epoch counters; built on the first such run after
     // an upload.
     golb200::ResidentBand* d_rjobs = nullptr;
-    uint32_t* d_rpub = nullptr;
-    int* d_rdone = nullptr;
-    int rjobs = 0, rdone = 0, rctas = 0;
+    unsigned long long* d_rpub = nullptr;
+    int rjobs = 0, rctas = 0;
     size_t rsmem = 0;
     golb200::ResidentBatchPlan rplan;
     double last_ms = 0;
@@ -832,12 +928,11 @@ int forced_band(const gol_batch::Entry& e) { return e.force_band ? e.force_band 
 void batch_free_device(gol_batch* b) {
     if (b->graph) cudaGraphExecDestroy(b->graph);
     b->graph = nullptr;
-    for (void* p : {(void*)b->d_rjobs, (void*)b->d_rpub, (void*)b->d_rdone})
+    for (void* p : {(void*)b->d_rjobs, (void*)b->d_rpub})
         if (p) cudaFree(p);
     b->d_rjobs = nullptr;
     b->d_rpub = nullptr;
-    b->d_rdone = nullptr;
-    b->rjobs = b->rdone = b->rctas = 0;
+    b->rjobs = b->rctas = 0;
     b->rsmem = 0;
     for (void* p : {(void*)b->arena, (void*)b->d_grids, (void*)b->d_items, (void*)b->d_done,
                     (void*)b->d_ticket, (void*)b->d_status, (void*)b->d_census, (void*)b->d_trk,
@@ -1216,20 +1311,18 @@ int gol_batch_run_resident(gol_batch* b) {
         if (const char* why = golb200::plan_resident_batch(rg.data(), rg.size(), b->num_sms,
                                                            b->device, &plan))
             return b->fail(GOL_E_UNSUPPORTED, why);
-        cudaError_t ce = cudaMalloc(&b->d_rpub, std::max<size_t>(plan.pub_words, 1) * sizeof(uint32_t));
-        if (ce == cudaSuccess) ce = cudaMalloc(&b->d_rdone, std::max(plan.ndone, 1) * sizeof(int));
+        cudaError_t ce = cudaMalloc(&b->d_rpub, std::max<size_t>(plan.pub_words, 1) * sizeof(unsigned long long));
         if (ce == cudaSuccess)
-            ce = cudaMalloc(&b->d_rjobs, std::max(plan.ndone, 1) * sizeof(golb200::ResidentBand));
+            ce = cudaMalloc(&b->d_rjobs, std::max(plan.nbands, 1) * sizeof(golb200::ResidentBand));
         if (ce != cudaSuccess) return b->cuda_fail(ce, "resident batch scratch");
-        std::vector<golb200::ResidentBand> jobs(plan.ndone);
-        golb200::fill_resident_jobs(plan, rg.data(), b->d_rpub, b->d_rdone, jobs.data());
+        std::vector<golb200::ResidentBand> jobs(plan.nbands);
+        golb200::fill_resident_jobs(plan, rg.data(), b->d_rpub, jobs.data());
         ce = cudaMemcpyAsync(b->d_rjobs, jobs.data(), jobs.size() * sizeof(golb200::ResidentBand),
                              cudaMemcpyHostToDevice, b->stream);
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(b->stream);
         if (ce != cudaSuccess) return b->cuda_fail(ce, "resident batch bands");
         b->rplan = plan;
-        b->rjobs = plan.ndone;
-        b->rdone = plan.ndone;
+        b->rjobs = plan.nbands;
         b->rctas = plan.ctas;
         b->rsmem = plan.smem;
     }
@@ -1240,7 +1333,7 @@ int gol_batch_run_resident(gol_batch* b) {
             ce = cudaMemcpyAsync(b->arena + e.offset + e.stride, b->arena + e.offset,
                                  (size_t)e.pitch * e.Y * sizeof(uint32_t), cudaMemcpyDeviceToDevice,
                                  b->stream);
-    if (ce == cudaSuccess) ce = cudaMemsetAsync(b->d_rdone, 0, std::max(b->rdone, 1) * sizeof(int), b->stream);
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(b->d_rpub, 0, std::max<size_t>(b->rplan.pub_words, 1) * sizeof(unsigned long long), b->stream);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(b->d_ticket, 0, sizeof(int), b->stream);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(b->d_status, 0, sizeof(int), b->stream);
     if (ce == cudaSuccess && b->rjobs)

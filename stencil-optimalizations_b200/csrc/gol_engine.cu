@@ -55,8 +55,8 @@ struct gol_engine {
     // shared-memory-resident run (GOL_ALG_RESIDENT)
     bool resident = false;
     golb200::ResidentPlan rplan{};
-    uint32_t* r_pub = nullptr;
-    int* r_ints = nullptr;                 // epoch counters, then the status word
+    unsigned long long* r_pub = nullptr;   // exchange slots
+    int* r_status = nullptr;
 
     // change tracking (GOL_ALG_LOCAL)
     bool local = false;
@@ -108,9 +108,9 @@ void release_device(gol_engine* e) {
     release_graphs(e);
     release_local(e);
     if (e->r_pub) cudaFree(e->r_pub);
-    if (e->r_ints) cudaFree(e->r_ints);
+    if (e->r_status) cudaFree(e->r_status);
     e->r_pub = nullptr;
-    e->r_ints = nullptr;
+    e->r_status = nullptr;
     for (auto& p : e->d) {
         if (p) cudaFree(p);
         p = nullptr;
@@ -442,8 +442,8 @@ int gol_init(gol_engine* e) {
         if (rc) return rc;
     }
     if (e->resident && !e->r_pub) {
-        ce = cudaMalloc(&e->r_pub, std::max<size_t>(e->rplan.pub_words, 1) * sizeof(uint32_t));
-        if (ce == cudaSuccess) ce = cudaMalloc(&e->r_ints, (e->rplan.nbands + 1) * sizeof(int));
+        ce = cudaMalloc(&e->r_pub, std::max<size_t>(e->rplan.pub_words, 1) * sizeof(unsigned long long));
+        if (ce == cudaSuccess) ce = cudaMalloc(&e->r_status, sizeof(int));
         if (ce != cudaSuccess) {
             release_device(e);
             return e->cuda_fail(ce, "resident-run scratch");
@@ -482,8 +482,8 @@ int gol_run(gol_engine* e, uint64_t n) {
             if (time_is_up()) return GOL_OK;
             const uint64_t chunk = std::min<uint64_t>(n - done, budget ? step : (1ull << 30));
             cudaError_t ce = golb200::launch_resident(e->d[e->cur], e->d[e->cur ^ 1], e->W, e->Y,
-                                                      (long long)chunk, e->rplan, e->r_pub, e->r_ints,
-                                                      e->r_ints + e->rplan.nbands, e->stream);
+                                                      (long long)chunk, e->rplan, e->r_pub, e->r_status,
+                                                      e->stream);
             if (ce == cudaSuccess && budget) ce = cudaStreamSynchronize(e->stream);
             if (ce != cudaSuccess) return e->cuda_fail(ce, "resident run launch");
             e->cur ^= 1;
@@ -557,9 +557,9 @@ int gol_run(gol_engine* e, uint64_t n) {
 // A resident run records GOL_E_TIMEOUT in its status word when a CTA gave
 // up waiting for a neighbour (bounded polls); reported after a sync.
 static int resident_status(gol_engine* e) {
-    if (!e->resident || !e->r_ints) return GOL_OK;
+    if (!e->resident || !e->r_status) return GOL_OK;
     int st = 0;
-    cudaError_t ce = cudaMemcpy(&st, e->r_ints + e->rplan.nbands, sizeof(int), cudaMemcpyDeviceToHost);
+    cudaError_t ce = cudaMemcpy(&st, e->r_status, sizeof(int), cudaMemcpyDeviceToHost);
     if (ce != cudaSuccess) return e->cuda_fail(ce, "resident status");
     return st ? e->fail(st, "a resident-run CTA gave up waiting for a neighbour") : GOL_OK;
 }
@@ -653,7 +653,7 @@ int gol_plan(const gol_engine* e, uint32_t* temporal_steps, uint32_t* band_rows,
     if (e->resident) {   // generations per epoch, the largest CTA band
         if (temporal_steps) *temporal_steps = (uint32_t)e->rplan.K;
         if (band_rows) *band_rows = (uint32_t)e->rplan.band;
-        if (words_per_lane) *words_per_lane = (uint32_t)e->rplan.wpl;
+        if (words_per_lane) *words_per_lane = 4;
         return GOL_OK;
     }
     if (temporal_steps) *temporal_steps = (uint32_t)e->k;

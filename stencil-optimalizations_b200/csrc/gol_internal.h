@@ -49,14 +49,12 @@ int best_depth(int W, int Y, int num_sms);
 struct ResidentBand {
     const uint32_t* src;   // the grid at generation 0 (row r at src + r * pitch)
     uint32_t* dst;         // the grid after `gens` generations (not src)
-    uint32_t* pub;         // the grid's exchange slots: band b's at (b * 4 + parity * 2 + side)
-                           // * K * ppitch words (side 0: its top K rows, 1: its bottom K rows)
-    int* done;             // the grid's epoch counters, one per band, zero at start
+    unsigned long long* pub;   // the grid's exchange slots, zero at start: band b's at (b * 4 + parity * 2 + side)
+                           // * K * 4 * lanes words (side 0: its top K rows, 1: its bottom K rows)
     int pitch;             // words from one grid row to the next (>= W)
-    int ppitch;            // words per row in the exchange slots (>= W, a multiple of 4)
     int W, Y;              // words per row, rows
     int K;                 // generations per epoch
-    int lanes, groups;     // threads: lanes across a row x row groups
+    int lanes, groups;     // threads: lanes of four words across a row x row groups
     int b, nb;             // this band, bands of the grid (rows split evenly)
     long long gens;
 };
@@ -76,13 +74,12 @@ struct ResidentGrid {
 struct ResidentBatchPlan {
     struct Grid {
         int index;             // into the ResidentGrid list
-        int nb, K, lanes, groups, ppitch;
+        int nb, K, lanes, groups;
         size_t pub_off;        // words into the exchange slots
-        int done_off;          // ints into the counters
     };
     std::vector<Grid> grids;
-    size_t smem = 0, pub_words = 0;
-    int ndone = 0;             // bands in all
+    size_t smem = 0, pub_words = 0;   // (64-bit words)
+    int nbands = 0;            // bands in all
     int ctas = 0;
 };
 // Plans grids g[0..n) (every gens > 0); nullptr or why they cannot run.
@@ -90,28 +87,28 @@ const char* plan_resident_batch(const ResidentGrid* g, size_t n, int num_sms, in
                                 ResidentBatchPlan* p);
 // Whether a W x Y grid can run in a resident batch (whatever its generations).
 bool resident_batch_fits(int W, int Y, int num_sms, int device);
-// The band list (p.ndone entries, launch order) given the slots and counters.
-void fill_resident_jobs(const ResidentBatchPlan& p, const ResidentGrid* g, uint32_t* pub, int* done,
+// The band list (p.nbands entries, launch order) given the slots.
+void fill_resident_jobs(const ResidentBatchPlan& p, const ResidentGrid* g, unsigned long long* pub,
                         ResidentBand* jobs);
 // One persistent cooperative launch over the bands; ticket, status and the
-// counters must be zero.
+// slots must be zero.
 cudaError_t launch_batch_resident(const ResidentBand* jobs, int njobs, int* ticket, int* status,
                                   const ResidentBatchPlan& p, cudaStream_t stream);
 
 struct ResidentPlan {
-    int wpl = 0, lanes = 0, groups = 0;   // lanes of wpl words across a row, row groups
+    int lanes = 0, groups = 0;            // lanes of four words across a row, row groups
     int K = 0;                            // generations per epoch (halo rows)
     int band = 0, nbands = 0;             // largest band, CTAs
     size_t smem = 0;                      // dynamic shared memory per CTA
-    size_t pub_words = 0;                 // words of the publication slots
+    size_t pub_words = 0;                 // (64-bit) words of the publication slots
 };
 // False when the grid does not fit (or k_epoch is out of range). k_epoch = 0
 // picks the default.
 bool plan_resident(int W, int Y, int k_epoch, int device, ResidentPlan* p);
-// gens generations src -> dst. pub (p.pub_words), epoch_done (p.nbands ints)
-// and status are device scratch; epoch_done and status are cleared here.
+// gens generations src -> dst. pub (p.pub_words) and status are device
+// scratch, cleared here.
 cudaError_t launch_resident(const uint32_t* src, uint32_t* dst, int W, int Y, long long gens,
-                            const ResidentPlan& p, uint32_t* pub, int* epoch_done, int* status,
+                            const ResidentPlan& p, unsigned long long* pub, int* status,
                             cudaStream_t stream, long long spin_limit = 0);
 
 // One pass of k generations (1 <= k <= kMaxKForWpl(plan.wpl)). pitch: words

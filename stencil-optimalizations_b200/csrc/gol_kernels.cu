@@ -235,21 +235,27 @@ bool plan_rows(int W, int Y, int k, int band_rows, int wpl, int num_sms, RowsPla
 #ifndef GOL_RESIDENT_K
 #define GOL_RESIDENT_K 8   // generations per epoch of the resident run
 #endif
-#ifndef GOL_RESIDENT_WPL
-#define GOL_RESIDENT_WPL 2
-#endif
 #ifndef GOL_RESIDENT_THREADS
 #define GOL_RESIDENT_THREADS 512   // threads per CTA (lanes across a row x row groups)
+#endif
+
+#ifndef GOL_RESIDENT_ROWS
+// Row groups are cut so that each has about this many rows or more (a group
+// reads two rows beside its own): 1 / 2 / 3 ran 1024 generations of 2048^2 in
+// 0.79 / 0.82 / 0.75 ms, of 3072 x 1024 in 0.84 / 0.80 / 0.99 ms.
+#define GOL_RESIDENT_ROWS 2
 #endif
 
 bool plan_resident(int W, int Y, int k_epoch, int device, ResidentPlan* p) {
     const int K = k_epoch > 0 ? k_epoch : GOL_RESIDENT_K;
     if (K < 1 || K > 64 || W <= 0 || Y <= 0) return false;
-    int wpl = GOL_RESIDENT_WPL;
-    while (wpl > 1 && W % wpl) wpl /= 2;
-    const int lanes = ((W + wpl - 1) / wpl + 31) / 32 * 32;
-    if (lanes > kResidentMaxThreads) return false;
-    const int groups = std::max(1, std::min(GOL_RESIDENT_THREADS, kResidentMaxThreads) / lanes);
+    const int lanes = (W + 3) / 4;
+    // The grids a resident run takes (gol_init refuses the others): rows of up
+    // to 1024 words, 512 when odd, and bands whose two buffers fit with rows
+    // of `accepted` words (the rows themselves are shorter).
+    const int unit = W % 2 ? 1 : 2;
+    const int accepted = (W / unit + 31) / 32 * 32 * unit + 8;
+    if ((W / unit + 31) / 32 * 32 > kResidentMaxThreads) return false;
     int sms = 0, smem_max = 0, coop = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
         cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess ||
@@ -260,58 +266,47 @@ bool plan_resident(int W, int Y, int k_epoch, int device, ResidentPlan* p) {
     // A grid of fewer than K rows is one band with no neighbours.
     const int nbands = std::max(1, std::min(sms, Y / K));
     const int band = (Y + nbands - 1) / nbands;
-    const size_t smem = resident_smem_bytes(band, K, lanes, wpl);
-    if (smem + 1024 > (size_t)smem_max) return false;
-    p->wpl = wpl;
+    if (2ull * (band + 2 * K) * accepted * sizeof(uint32_t) + 1024 > (size_t)smem_max) return false;
+    const size_t smem = resident_smem_bytes(band, K, lanes);
     p->lanes = lanes;
-    p->groups = groups;
+    p->groups = std::max(1, std::min(std::min(GOL_RESIDENT_THREADS, kResidentMaxThreads) / lanes,
+                                     (band + K + GOL_RESIDENT_ROWS - 1) / GOL_RESIDENT_ROWS));
     p->K = K;
     p->band = band;
     p->nbands = nbands;
     p->smem = smem;
-    p->pub_words = (size_t)nbands * 4 * K * W;
+    p->pub_words = (size_t)nbands * 4 * K * 4 * lanes;
     return true;
 }
 
-template <int WPL, int LANES>
+template <int LANES>
 static cudaError_t launch_resident_lanes(const ResidentLaunch& a, const ResidentPlan& p,
                                          cudaStream_t stream) {
-    cudaError_t e = cudaFuncSetAttribute(rows_resident_kernel<WPL, LANES>,
+    cudaError_t e = cudaFuncSetAttribute(rows_resident_kernel<LANES>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
     if (e != cudaSuccess) return e;
     ResidentLaunch arg = a;
     void* args[] = {&arg};
-    return cudaLaunchCooperativeKernel((const void*)rows_resident_kernel<WPL, LANES>,
-                                       dim3(p.nbands), dim3(p.lanes * p.groups), args, p.smem,
+    // whole warps: the threads past the last row group are idle in the passes
+    return cudaLaunchCooperativeKernel((const void*)rows_resident_kernel<LANES>, dim3(p.nbands),
+                                       dim3((p.lanes * p.groups + 31) / 32 * 32), args, p.smem,
                                        stream);
 }
 
-// Row widths of 64, 128 and 256 lanes (4096-, 8192- and 16384-cell rows at
-// two words per lane) get a compile-time row stride; others a runtime one.
-template <int WPL>
-static cudaError_t launch_resident_wpl(const ResidentLaunch& a, const ResidentPlan& p,
-                                       cudaStream_t stream) {
-    switch (p.lanes) {
-        case 64: return launch_resident_lanes<WPL, 64>(a, p, stream);
-        case 128: return launch_resident_lanes<WPL, 128>(a, p, stream);
-        case 256: return launch_resident_lanes<WPL, 256>(a, p, stream);
-        default: return launch_resident_lanes<WPL, 0>(a, p, stream);
-    }
-}
-
 cudaError_t launch_resident(const uint32_t* src, uint32_t* dst, int W, int Y, long long gens,
-                            const ResidentPlan& p, uint32_t* pub, int* epoch_done, int* status,
+                            const ResidentPlan& p, unsigned long long* pub, int* status,
                             cudaStream_t stream, long long spin_limit) {
-    cudaError_t e = cudaMemsetAsync(epoch_done, 0, (size_t)p.nbands * sizeof(int), stream);
+    cudaError_t e = cudaMemsetAsync(pub, 0, p.pub_words * sizeof(unsigned long long), stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(status, 0, sizeof(int), stream);
     if (e != cudaSuccess) return e;
-    ResidentLaunch a{src, dst, pub, epoch_done, status, W, Y, p.K, p.lanes, p.groups, gens,
+    ResidentLaunch a{src, dst, pub, status, W, Y, p.K, p.lanes, p.groups, gens,
                      spin_limit > 0 ? spin_limit : (1ll << 24)};
-    switch (p.wpl) {
-        case 4: return launch_resident_wpl<4>(a, p, stream);
-        case 2: return launch_resident_wpl<2>(a, p, stream);
-        case 1: return launch_resident_wpl<1>(a, p, stream);
-        default: return cudaErrorInvalidValue;
+    // Rows of 4096, 8192 and 16384 cells get a compile-time row stride.
+    switch (p.lanes) {
+        case 32: return launch_resident_lanes<32>(a, p, stream);
+        case 64: return launch_resident_lanes<64>(a, p, stream);
+        case 128: return launch_resident_lanes<128>(a, p, stream);
+        default: return launch_resident_lanes<0>(a, p, stream);
     }
 }
 

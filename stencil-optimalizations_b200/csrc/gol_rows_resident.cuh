@@ -21,18 +21,29 @@
 // K - g halo rows each side that the halo still determines). Rows outside
 // the grid are never computed and stay dead (zero).
 //
-// Epoch e publishes the band's top and bottom K rows into slot e & 1 and
-// releases an epoch counter; a CTA rewrites a slot two epochs later, after
-// both neighbours have published the epoch in between, i.e. after they read
-// it.
+// Epoch e publishes the band's top and bottom K rows into slot e & 1, every
+// word with the epoch's tag e + 1 beside it in one 64-bit store: the
+// neighbours poll the words themselves, so an exchange costs one trip through
+// L2 and no fence, counter or barrier of its own (the slots are zeroed before
+// a launch). A CTA rewrites a slot two epochs later, after both neighbours
+// have published the epoch in between, i.e. after they read it.
 //
-// Within a pass a thread owns WPL words of a column (the CTA's threads are
-// lanes across the row times row groups) and walks a range of rows with
-// the horizontal sums of three rows in registers. Shared-memory rows carry
-// four zero words of padding each side, so the words just outside a lane's
-// span are plain loads from the row (cheaper on the integer pipe, the
-// bound here, than shuffles and selects). Columns at or past W exist only
-// in the last lanes of a row, which alone run the masked variant.
+// Within a pass a thread owns four words of a row (128 cells; the CTA's
+// threads are lanes across the row times row groups) and walks a range of
+// rows two at a time (pair_sum, next_word_pair in gol_word_ops.cuh), the sums
+// of the two rows above in registers. The run is bound by the integer pipe,
+// so shared memory holds the lane's cells interleaved: bit i of its word j is
+// cell 4i + j. The cells left and right of a word's are then the words before
+// and after it, and only the outer two neighbours of a lane's four words take
+// a shift: 8.5 operations a word and generation, against 12 for rows as they
+// are, one at a time (9.4 -> 6.5 ms for 8192^2, 4096 generations). A band is
+// interleaved when it is loaded and restored when it is stored, some 8
+// operations a word each way; the exchange slots hold interleaved rows. The
+// four words are kept in planes (word j of all lanes in a run), so every
+// access takes one wavefront: ten for a warp's 128 words of a row, where the
+// integer pipe takes 17 cycles. (With the four words of a lane side by side
+// the two neighbour loads alone take eight.) Cells at or past column W are
+// masked by the warps that hold some.
 //
 // The band algorithm (resident_band) serves two kernels: one grid, CTA c
 // running band c (rows_resident_kernel), and many grids, persistent CTAs
@@ -53,7 +64,6 @@ namespace golb200 {
 #define GOL_RESIDENT_MAX_THREADS 512
 #endif
 constexpr int kResidentMaxThreads = GOL_RESIDENT_MAX_THREADS;
-constexpr int kResidentPad = 4;   // zero words each side of a shared-memory row
 #ifndef GOL_RESIDENT_INTERIOR
 #define GOL_RESIDENT_INTERIOR 1
 #endif
@@ -64,185 +74,219 @@ constexpr int kResidentInterior = GOL_RESIDENT_INTERIOR;
 struct ResidentLaunch {   // one grid (rows_resident_kernel)
     const uint32_t* src;   // the grid at generation 0 (W words per row, Y rows)
     uint32_t* dst;         // the grid after `gens` generations (not src)
-    uint32_t* pub;         // [nbands][2 parities][2 sides][K rows][W words]
-    int* epoch_done;       // [nbands], zero at launch: epochs published
+    unsigned long long* pub;   // [nbands][2 parities][2 sides][K rows][4 planes][lanes], zero at launch
     int* status;           // GOL_E_TIMEOUT if a wait gave up
     int W, Y;
     int K;                 // generations per epoch
-    int lanes;             // lanes across a row (ceil(W / WPL), a multiple of 32)
+    int lanes;             // lanes across a row, four words each: ceil(W / 4)
     int groups;            // row groups (blockDim.x = lanes * groups)
     long long gens;
     long long spin_limit;
 };
 
-__device__ __forceinline__ int ld_acquire_gpu(const int* p) {
-    int v;
-    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+// A published word: the value below, the epoch's tag above, stored and loaded
+// at once.
+__device__ __forceinline__ void st_tagged(unsigned long long* p, uint32_t v, uint32_t tag) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"((unsigned long long)tag << 32 | v)
+                 : "memory");
+}
+
+__device__ __forceinline__ unsigned long long ld_tagged(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
 
-__device__ __forceinline__ void st_release_gpu(int* p, int v) {
-    asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+// A shared-memory row: a zero word, plane 3 of the lanes, planes 1 and 2,
+// plane 0, a zero word. The words beyond a row's ends that a pass reads are
+// plane 3 before lane 0 and plane 0 after the last lane: the zero words. Rows
+// whose lanes do not fill warps have an odd stride, so that the row groups of
+// one warp fall into different banks.
+__host__ __device__ inline int resident_stride(int lanes) {
+    return 4 * lanes + 2 + (lanes % 32 ? 1 : 0);
 }
-
-// Words per shared-memory row: the lanes' words plus the padding.
-__host__ __device__ inline int resident_stride(int lanes, int wpl) {
-    return lanes * wpl + 2 * kResidentPad;
-}
+__host__ __device__ constexpr int resident_plane(int j) { return j == 3 ? 0 : j == 0 ? 3 : j; }
 
 // Shared memory of one CTA: two buffers of (band + 2K) rows.
-__host__ __device__ inline size_t resident_smem_bytes(int band, int K, int lanes, int wpl) {
-    return 2ull * (size_t)(band + 2 * K) * (size_t)resident_stride(lanes, wpl) * sizeof(uint32_t);
+__host__ __device__ inline size_t resident_smem_bytes(int band, int K, int lanes) {
+    return 2ull * (size_t)(band + 2 * K) * (size_t)resident_stride(lanes) * sizeof(uint32_t);
 }
 
-template <int WPL>
-__device__ __forceinline__ void lds_words_gen(const uint32_t* p, uint32_t (&v)[WPL]) {
-    if constexpr (WPL == 4) {
-        const uint4 t = *reinterpret_cast<const uint4*>(p);
-        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-    } else if constexpr (WPL == 2) {
-        const uint2 t = *reinterpret_cast<const uint2*>(p);
-        v[0] = t.x; v[1] = t.y;
-    } else {
-        v[0] = *p;
-    }
-}
-
-template <int WPL>
-__device__ __forceinline__ void sts_words_gen(uint32_t* p, const uint32_t (&v)[WPL]) {
-    if constexpr (WPL == 4) {
-        *reinterpret_cast<uint4*>(p) = make_uint4(v[0], v[1], v[2], v[3]);
-    } else if constexpr (WPL == 2) {
-        *reinterpret_cast<uint2*>(p) = make_uint2(v[0], v[1]);
-    } else {
-        *p = v[0];
-    }
-}
-
-// A lane's WPL words from global memory through L2 only (the exchange
-// slots, which other CTAs rewrite).
-template <int WPL>
-__device__ __forceinline__ void ldcg_words(const uint32_t* p, uint32_t (&v)[WPL]) {
-    if constexpr (WPL == 4) {
-        const uint4 t = __ldcg(reinterpret_cast<const uint4*>(p));
-        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-    } else if constexpr (WPL == 2) {
-        const uint2 t = __ldcg(reinterpret_cast<const uint2*>(p));
-        v[0] = t.x; v[1] = t.y;
-    } else {
-        v[0] = __ldcg(p);
-    }
-}
-
-// Horizontal sums of the shared-memory row at p (this lane's words). The
-// words just outside the lane's span are plain loads from the row (its
-// neighbours' words, or the zero padding at the row's ends): no shuffles,
-// selects or divergent loads.
-template <int WPL>
-__device__ __forceinline__ void resident_hsum(const uint32_t* p, uint32_t (&c)[WPL],
-                                              uint32_t (&h0)[WPL], uint32_t (&h1)[WPL]) {
-    lds_words_gen<WPL>(p, c);
-    const uint32_t lw = p[-1];
-    const uint32_t rw = p[WPL];
+// Exchanges index bit B of the bit position with the upper bit of the register
+// index (v[0], v[1] against v[2], v[3]).
+template <int B>
+__device__ __forceinline__ void swap_index_bit(uint32_t (&v)[4]) {
+    constexpr uint32_t m = B == 4 ? 0x0000ffffu : B == 3 ? 0x00ff00ffu : B == 2 ? 0x0f0f0f0fu
+                           : B == 1 ? 0x33333333u : 0x55555555u;   // positions whose bit B is 0
 #pragma unroll
-    for (int w = 0; w < WPL; ++w) {
-        const uint32_t l = w == 0 ? lw : c[w - 1];
-        const uint32_t r = w == WPL - 1 ? rw : c[w + 1];
-        hsum(l, c[w], r, h0[w], h1[w]);
+    for (int i = 0; i < 2; ++i) {
+        const uint32_t x = v[i], y = v[i + 2];
+        v[i] = (x & m) | ((y & m) << (1 << B));
+        v[i + 2] = ((x >> (1 << B)) & m) | (y & ~m);
     }
 }
 
-// One output row from the ring slots M (above), C (the row) and P (below).
-template <int WPL, bool RAG, int M, int C, int P>
-__device__ __forceinline__ void resident_row(const uint32_t (&h0)[3][WPL],
-                                             const uint32_t (&h1)[3][WPL],
-                                             const uint32_t (&cw)[3][WPL], uint32_t* d,
-                                             const uint32_t (&cm)[WPL]) {
-    uint32_t res[WPL];
+__device__ __forceinline__ void swap_registers(uint32_t (&v)[4]) {   // the register index's two bits
+    const uint32_t t = v[1];
+    v[1] = v[2];
+    v[2] = t;
+}
+
+// Cell c of the lane's 128 from bit c % 32 of word c / 32 to bit c / 4 of word
+// c % 4, and back: the index (w1 w0 a2 a1 a0 j1 j0) rotated by two, one bit
+// at a time through the register index.
+__device__ __forceinline__ void interleave4(uint32_t (&v)[4]) {
+    swap_index_bit<4>(v);
+    swap_index_bit<2>(v);
+    swap_index_bit<0>(v);
+    swap_registers(v);
+    swap_index_bit<3>(v);
+    swap_index_bit<1>(v);
+}
+
+__device__ __forceinline__ void deinterleave4(uint32_t (&v)[4]) {
+    swap_index_bit<1>(v);
+    swap_index_bit<3>(v);
+    swap_registers(v);
+    swap_index_bit<0>(v);
+    swap_index_bit<2>(v);
+    swap_index_bit<4>(v);
+}
+
+// One row of a lane: its four words, and their horizontal sums.
+struct ResidentRow {
+    uint32_t c[4], h0[4], h1[4];
+};
+
+// Reads the row whose first plane's entry of this lane is at p (planes PL
+// words apart).
+__device__ __forceinline__ void resident_row(const uint32_t* p, int PL, ResidentRow& r) {
 #pragma unroll
-    for (int w = 0; w < WPL; ++w) {
-        res[w] = next_word(h0[M][w], h1[M][w], h0[C][w], h1[C][w], h0[P][w], h1[P][w], cw[C][w]);
-        if constexpr (RAG) res[w] &= cm[w];
+    for (int j = 0; j < 4; ++j) r.c[j] = p[resident_plane(j) * PL];
+    const uint32_t lw = p[-1];           // plane 3 of the lane before
+    const uint32_t rw = p[3 * PL + 1];   // plane 0 of the lane after
+    const uint32_t left = __funnelshift_l(lw, r.c[3], 1);
+    const uint32_t right = __funnelshift_r(r.c[0], rw, 1);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t l = j == 0 ? left : r.c[j - 1];
+        const uint32_t q = j == 3 ? right : r.c[j + 1];
+        r.h0[j] = lop3<LUT_XOR3>(l, r.c[j], q);
+        r.h1[j] = lop3<LUT_MAJ>(l, r.c[j], q);
     }
-    sts_words_gen<WPL>(d, res);
 }
 
-// Rows [r0, r1) of one generation, S -> D (S and D point at this lane's
-// first word of row 0). The loop body covers three rows so the ring slots
-// are compile-time register names; it has no early exits, so the loads of
-// its three rows can be issued together.
-template <int WPL, bool RAG>
+// The next state of rows b and p (a above b, q below p), to d and d + stride.
+template <bool RAG>
+__device__ __forceinline__ void resident_pair(const ResidentRow& a, const ResidentRow& b,
+                                              const ResidentRow& p, const ResidentRow& q,
+                                              uint32_t* d, int stride, int PL, uint32_t mask) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const PairSum s = pair_sum(b.h0[j], b.h1[j], p.h0[j], p.h1[j]);
+        uint32_t x = next_word_pair(a.h0[j], a.h1[j], s, b.c[j]);
+        uint32_t y = next_word_pair(q.h0[j], q.h1[j], s, p.c[j]);
+        if (RAG) {
+            x &= mask;
+            y &= mask;
+        }
+        d[resident_plane(j) * PL] = x;
+        d[stride + resident_plane(j) * PL] = y;
+    }
+}
+
+// Rows [r0, r1) of one generation, S -> D (S and D point at this lane's entry
+// of row 0's first plane). Four rows per turn, so that the rows' sums change
+// roles by name.
+template <bool RAG>
 __device__ __forceinline__ void resident_rows(const uint32_t* S, uint32_t* D, int r0, int r1,
-                                              int stride, const uint32_t (&cm)[WPL]) {
+                                              int stride, int PL, uint32_t mask) {
     if (r0 >= r1) return;
-    uint32_t h0[3][WPL], h1[3][WPL], cw[3][WPL];
+    ResidentRow a, b, p, q;
     const uint32_t* s = S + (size_t)(r0 - 1) * stride;
     uint32_t* d = D + (size_t)r0 * stride;
-    resident_hsum<WPL>(s, cw[0], h0[0], h1[0]);
-    s += stride;
-    resident_hsum<WPL>(s, cw[1], h0[1], h1[1]);
-    s += stride;
+    resident_row(s, PL, a);
+    resident_row(s + stride, PL, b);
+    s += 2 * stride;
     int n = r1 - r0;
-    for (; n >= 3; n -= 3) {   // slot 0: row r - 1, slot 1: row r
-        resident_hsum<WPL>(s, cw[2], h0[2], h1[2]);
-        resident_row<WPL, RAG, 0, 1, 2>(h0, h1, cw, d, cm);
-        resident_hsum<WPL>(s + stride, cw[0], h0[0], h1[0]);
-        resident_row<WPL, RAG, 1, 2, 0>(h0, h1, cw, d + stride, cm);
-        resident_hsum<WPL>(s + 2 * stride, cw[1], h0[1], h1[1]);
-        resident_row<WPL, RAG, 2, 0, 1>(h0, h1, cw, d + 2 * stride, cm);
-        s += 3 * stride;
-        d += 3 * stride;
+    for (; n >= 4; n -= 4) {
+        resident_row(s, PL, p);
+        resident_row(s + stride, PL, q);
+        resident_pair<RAG>(a, b, p, q, d, stride, PL, mask);
+        resident_row(s + 2 * stride, PL, a);
+        resident_row(s + 3 * stride, PL, b);
+        resident_pair<RAG>(p, q, a, b, d + 2 * stride, stride, PL, mask);
+        s += 4 * stride;
+        d += 4 * stride;
     }
-    if (n >= 1) {
-        resident_hsum<WPL>(s, cw[2], h0[2], h1[2]);
-        resident_row<WPL, RAG, 0, 1, 2>(h0, h1, cw, d, cm);
+    if (n >= 2) {
+        resident_row(s, PL, p);
+        resident_row(s + stride, PL, q);
+        resident_pair<RAG>(a, b, p, q, d, stride, PL, mask);
+        a = p;
+        b = q;
+        s += 2 * stride;
+        d += 2 * stride;
+        n -= 2;
     }
-    if (n == 2) {
-        resident_hsum<WPL>(s + stride, cw[0], h0[0], h1[0]);
-        resident_row<WPL, RAG, 1, 2, 0>(h0, h1, cw, d + stride, cm);
+    if (n == 1) {   // one row: its pair's other half is not wanted
+        resident_row(s, PL, p);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const PairSum x = pair_sum(b.h0[j], b.h1[j], p.h0[j], p.h1[j]);
+            uint32_t y = next_word_pair(a.h0[j], a.h1[j], x, b.c[j]);
+            if (RAG) y &= mask;
+            d[resident_plane(j) * PL] = y;
+        }
     }
 }
 
 // Rows [lo, hi) split over groups [g0, g0 + ng) (this thread's group is g).
-template <int WPL, bool RAG>
-__device__ __forceinline__ void resident_range(const uint32_t* S, uint32_t* D, int lo, int hi,
-                                               int g, int g0, int ng, int stride,
-                                               const uint32_t (&cm)[WPL]) {
-    if (g < g0 || g >= g0 + ng || hi <= lo) return;
-    const int per = (hi - lo + ng - 1) / ng;
-    const int r0 = lo + (g - g0) * per;
-    resident_rows<WPL, RAG>(S, D, r0, min(hi, r0 + per), stride, cm);
-}
-
-template <int WPL>
+// Rows of whole warps are split evenly: sizes differ by at most one row, so
+// the schedulers' shares do not drift apart (whole pairs per group left two of
+// them 10 % more). Narrower ones, several groups to a warp, lie as many rows
+// apart, and with the odd stride they share banks where that number has more
+// factors of two than the lanes: then they take a row more (256 x 2048: 12.7
+// thousand cycles a generation without, 4.4 with).
 __device__ __forceinline__ void resident_pass(const uint32_t* S, uint32_t* D, int lo, int hi,
-                                              int g, int g0, int ng, int stride,
-                                              const uint32_t (&cm)[WPL], bool rag) {
+                                              int g, int g0, int ng, int stride, int PL,
+                                              uint32_t mask, bool rag) {
+    if (g < g0 || g >= g0 + ng || hi <= lo) return;
+    const int n = hi - lo;
+    int r0, r1;
+    if (PL >= 32) {
+        const int q = n / ng, extra = n - q * ng;   // the first `extra` groups one more
+        r0 = lo + (g - g0) * q + min(g - g0, extra);
+        r1 = r0 + q + (g - g0 < extra ? 1 : 0);
+    } else {
+        int q = (n + ng - 1) / ng;
+        if (q % (2 * (PL & -PL)) == 0) ++q;
+        r0 = lo + (g - g0) * q;
+        r1 = min(hi, r0 + q);
+    }
     if (rag)   // the same for every lane of a warp
-        resident_range<WPL, true>(S, D, lo, hi, g, g0, ng, stride, cm);
+        resident_rows<true>(S, D, r0, r1, stride, PL, mask);
     else
-        resident_range<WPL, false>(S, D, lo, hi, g, g0, ng, stride, cm);
+        resident_rows<false>(S, D, r0, r1, stride, PL, mask);
 }
 
-// Global <-> register copies of a lane's words: vector accesses where the
-// lane's words are whole and aligned, else word by word up to W.
-template <int WPL>
-__device__ __forceinline__ void band_load(const uint32_t* p, bool vec, int n, uint32_t (&v)[WPL]) {
+// Global <-> register copies of a lane's four words: vector accesses where
+// they are whole and aligned, else word by word up to W.
+__device__ __forceinline__ void band_load(const uint32_t* p, bool vec, int n, uint32_t (&v)[4]) {
     if (vec) {
-        load_words<WPL>(p, v);
+        load_words<4>(p, v);
     } else {
 #pragma unroll
-        for (int w = 0; w < WPL; ++w) v[w] = w < n ? __ldg(p + w) : 0u;
+        for (int w = 0; w < 4; ++w) v[w] = w < n ? __ldg(p + w) : 0u;
     }
 }
 
-template <int WPL>
-__device__ __forceinline__ void band_store(uint32_t* p, bool vec, int n, const uint32_t (&v)[WPL]) {
+__device__ __forceinline__ void band_store(uint32_t* p, bool vec, int n, const uint32_t (&v)[4]) {
     if (vec) {
-        store_words<WPL>(p, v);
+        store_words<4>(p, v);
     } else {
 #pragma unroll
-        for (int w = 0; w < WPL; ++w)
+        for (int w = 0; w < 4; ++w)
             if (w < n) p[w] = v[w];
     }
 }
@@ -252,134 +296,134 @@ __device__ __forceinline__ void band_store(uint32_t* p, bool vec, int n, const u
 // smem holds 2 * (B + 2K) rows of the stride. LANES: the lanes across a row
 // when known at compile time (0: j.lanes), so the shared-memory row stride
 // is a constant and row addresses are immediate offsets.
-template <int WPL, int LANES>
+template <int LANES>
 __device__ __forceinline__ bool resident_band(const ResidentBand& j, uint32_t* smem, int* stop,
                                               int* status, long long spin_limit) {
     const int K = j.K;
-    const int stride = LANES ? resident_stride(LANES, WPL) : resident_stride(j.lanes, WPL);
-    const int lane_in_row = threadIdx.x % j.lanes;
-    const int group = threadIdx.x / j.lanes;   // >= j.groups: idle in the passes
-    const int col = lane_in_row * WPL;
+    const int PL = LANES ? LANES : j.lanes;
+    const int stride = resident_stride(PL);
+    const int lane_in_row = threadIdx.x % PL;
+    const int group = threadIdx.x / PL;   // >= j.groups: idle in the passes
+    const int col = lane_in_row * 4;
     const int W = j.W;
-    // Warps whose span reaches column W mask their results past it (when
-    // lanes is a multiple of 32 a warp lies within one row).
-    const bool rag = (j.lanes & 31) ? col + WPL > W : (lane_in_row | 31) * WPL + WPL > W;
-    uint32_t cm[WPL];
-#pragma unroll
-    for (int w = 0; w < WPL; ++w) cm[w] = col + w < W ? 0xffffffffu : 0u;
+    const int nw = W - col;               // words of this lane inside the row
+    // Warps with cells past column W mask their results: word j holds cells
+    // 4i + j, so a lane of nw words keeps the lower 8 nw bits of each.
+    const uint32_t mask = nw >= 4 ? 0xffffffffu : (1u << (8 * max(nw, 0))) - 1u;
+    const bool rag = __any_sync(0xffffffffu, mask != 0xffffffffu);
     const bool top = j.b == 0, bottom = j.b == j.nb - 1;
     // Bands split the rows evenly (sizes differ by at most one row; with
     // several bands every band is at least K rows).
     const int y0 = (int)((long long)j.b * j.Y / j.nb);
     const int B = (int)((long long)(j.b + 1) * j.Y / j.nb) - y0;
     const int rows = B + 2 * K;                 // shared-memory rows: K halo each side
-    const size_t side_words = (size_t)K * j.ppitch;
+    const size_t side_words = (size_t)K * 4 * PL;
     const int ng_top = j.groups > 1 ? j.groups / 2 : 1;
     const int g_bot = j.groups > 1 ? ng_top : 0;
     const int ng_bot = j.groups > 1 ? j.groups - ng_top : 1;
-    const bool mine_lane = col < W && group < j.groups;   // moves words between global and shared
-    const int nw = W - col;                             // words of this lane inside the row
-    const bool gvec = col + WPL <= W && (j.pitch % WPL) == 0;
+    const bool mover = group < j.groups;        // moves words between global and shared
+    const bool whole = nw >= 4 && (j.pitch & 3) == 0;
+    const bool svec = whole && ((uintptr_t)j.src & 15u) == 0;
+    const bool dvec = whole && ((uintptr_t)j.dst & 15u) == 0;
 
-    // Buffers zero (halo rows, padding, columns past W), then the band rows
+    // Buffers zero (halo rows, the rows' outer words), then the band rows
     // into buffer 0 (shared row K + i = grid row y0 + i). Copies between
     // global and shared rows go by row group and lane: each thread moves its
-    // lane's WPL words of every groups-th row.
+    // lane's four words of every groups-th row.
     for (int i = threadIdx.x; i < 2 * rows * stride; i += blockDim.x) smem[i] = 0u;
     __syncthreads();
-    uint32_t* const lane0w = smem + kResidentPad + col;   // this lane's words of shared row 0
-    if (mine_lane) {
+    uint32_t* const lane0 = smem + 1 + lane_in_row;   // this lane's entry of row 0's first plane
+    if (mover) {
         for (int r = group; r < B; r += j.groups) {
-            uint32_t v[WPL];
-            band_load<WPL>(j.src + (size_t)(y0 + r) * j.pitch + col, gvec, nw, v);
-            sts_words_gen<WPL>(lane0w + (size_t)(K + r) * stride, v);
+            uint32_t v[4];
+            band_load(j.src + (size_t)(y0 + r) * j.pitch + col, svec, nw, v);
+            interleave4(v);
+            uint32_t* d = lane0 + (size_t)(K + r) * stride;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) d[resident_plane(i) * PL] = v[i];
         }
     }
     if (threadIdx.x == 0) *stop = 0;
     __syncthreads();
 
-    const uint32_t* const lane0 = lane0w;
     int cur = 0;
     long long left = j.gens;
     for (int e = 0; left > 0; ++e) {
         const int kk = (int)min((long long)K, left);
         // Publish the band's top and bottom K rows (the state at epoch start).
-        uint32_t* mine = j.pub + ((size_t)j.b * 4 + (e & 1) * 2) * side_words + col;
-        const uint32_t* Aw = lane0w + (cur ? (size_t)rows * stride : 0);
-        if (mine_lane) {
+        const uint32_t tag = (uint32_t)e + 1u;
+        unsigned long long* mine = j.pub + ((size_t)j.b * 4 + (e & 1) * 2) * side_words + lane_in_row;
+        uint32_t* const Aw = lane0 + (cur ? (size_t)rows * stride : 0);
+        if (mover) {
             for (int r = group; r < K; r += j.groups) {
-                uint32_t v[WPL];
-                if (!top) {
-                    lds_words_gen<WPL>(Aw + (size_t)(K + r) * stride, v);
-                    store_words<WPL>(mine + (size_t)r * j.ppitch, v);
-                }
-                if (!bottom) {
-                    lds_words_gen<WPL>(Aw + (size_t)(B + r) * stride, v);
-                    store_words<WPL>(mine + side_words + (size_t)r * j.ppitch, v);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const size_t at = ((size_t)r * 4 + i) * PL;
+                    if (!top) st_tagged(mine + at, Aw[(size_t)(K + r) * stride + i * PL], tag);
+                    if (!bottom)
+                        st_tagged(mine + side_words + at, Aw[(size_t)(B + r) * stride + i * PL], tag);
                 }
             }
         }
-        __syncthreads();
-        if (threadIdx.x == 0) st_release_gpu(j.done + j.b, e + 1);
         // The interior: generation g's rows at least g from the band's edges,
         // for the first ni generations (enough to cover the exchange).
         const int ni = min(kk, kResidentInterior);
         for (int g = 1; g <= ni; ++g) {
             const int sb = (cur + g - 1) & 1;
             const uint32_t* S = lane0 + (sb ? (size_t)rows * stride : 0);
-            uint32_t* D = const_cast<uint32_t*>(lane0) + (sb ? 0 : (size_t)rows * stride);
-            resident_pass<WPL>(S, D, K + g, K + B - g, group, 0, j.groups, stride, cm, rag);
+            uint32_t* D = lane0 + (sb ? 0 : (size_t)rows * stride);
+            resident_pass(S, D, K + g, K + B - g, group, 0, j.groups, stride, PL, mask, rag);
             __syncthreads();
         }
-        // Wait for the neighbours' rows of this epoch (bounded).
-        if (threadIdx.x < 2) {
-            const int nb = threadIdx.x == 0 ? j.b - 1 : j.b + 1;
-            if (nb >= 0 && nb < j.nb) {
+        // The neighbours' rows of this epoch, polled word by word (bounded):
+        // the upper one's bottom rows, the lower one's top rows. At the grid's
+        // edges the halo stays zero (never written).
+        if (mover) {
+            const unsigned long long* up =
+                j.pub + ((size_t)(j.b - 1) * 4 + (e & 1) * 2 + 1) * side_words + lane_in_row;
+            const unsigned long long* dn =
+                j.pub + ((size_t)(j.b + 1) * 4 + (e & 1) * 2) * side_words + lane_in_row;
+            for (int r = group; r < K; r += j.groups) {
+                unsigned long long u[4], v[4];
                 long long spins = 0;
-                while (ld_acquire_gpu(j.done + nb) < e + 1) {
+                for (;;) {
+                    bool here = true;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const size_t at = ((size_t)r * 4 + i) * PL;
+                        u[i] = top ? (unsigned long long)tag << 32 : ld_tagged(up + at);
+                        v[i] = bottom ? (unsigned long long)tag << 32 : ld_tagged(dn + at);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        here = here && (uint32_t)(u[i] >> 32) == tag && (uint32_t)(v[i] >> 32) == tag;
+                    if (here) break;
                     if (++spins > spin_limit || *(volatile int*)status != 0) {
                         atomicCAS(status, 0, GOL_E_TIMEOUT);
                         atomicExch(stop, 1);
                         break;
                     }
-                    __nanosleep(64);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (!top) Aw[(size_t)r * stride + i * PL] = (uint32_t)u[i];
+                    if (!bottom) Aw[(size_t)(K + B + r) * stride + i * PL] = (uint32_t)v[i];
                 }
             }
         }
         __syncthreads();
         if (*(volatile int*)stop) return false;   // the same for every thread of the CTA
-        // Halo rows: the upper neighbour's bottom rows, the lower one's top
-        // rows, loaded from L2 (a slot is rewritten every other epoch, so no
-        // copy of it may linger in L1). At the grid's edges they stay zero
-        // (never written).
-        if (mine_lane) {
-            const uint32_t* up = j.pub + ((size_t)(j.b - 1) * 4 + (e & 1) * 2 + 1) * side_words + col;
-            const uint32_t* dn = j.pub + ((size_t)(j.b + 1) * 4 + (e & 1) * 2) * side_words + col;
-            uint32_t* Aw2 = lane0w + (cur ? (size_t)rows * stride : 0);
-            for (int r = group; r < K; r += j.groups) {
-                uint32_t v[WPL];
-                if (!top) {
-                    ldcg_words<WPL>(up + (size_t)r * j.ppitch, v);
-                    sts_words_gen<WPL>(Aw2 + (size_t)r * stride, v);
-                }
-                if (!bottom) {
-                    ldcg_words<WPL>(dn + (size_t)r * j.ppitch, v);
-                    sts_words_gen<WPL>(Aw2 + (size_t)(K + B + r) * stride, v);
-                }
-            }
-        }
-        __syncthreads();
         // Generations 1..ni near the edges: rows within g of the band's
         // edges, and the halo rows the later generations still need.
         for (int g = 1; g <= ni; ++g) {
             const int sb = (cur + g - 1) & 1;
             const uint32_t* S = lane0 + (sb ? (size_t)rows * stride : 0);
-            uint32_t* D = const_cast<uint32_t*>(lane0) + (sb ? 0 : (size_t)rows * stride);
+            uint32_t* D = lane0 + (sb ? 0 : (size_t)rows * stride);
             const int bhi = bottom ? K + B : K + B + kk - g;
             const int tlo = top ? K : K - kk + g, thi = min(K + g, bhi);   // (a band under g rows)
             const int blo = max(K + g, K + B - g);
-            resident_pass<WPL>(S, D, tlo, thi, group, 0, ng_top, stride, cm, rag);
-            resident_pass<WPL>(S, D, blo, bhi, group, g_bot, ng_bot, stride, cm, rag);
+            resident_pass(S, D, tlo, thi, group, 0, ng_top, stride, PL, mask, rag);
+            resident_pass(S, D, blo, bhi, group, g_bot, ng_bot, stride, PL, mask, rag);
             __syncthreads();
         }
         // Generations ni+1..kk whole: the band and what the halo still
@@ -387,28 +431,30 @@ __device__ __forceinline__ bool resident_band(const ResidentBand& j, uint32_t* s
         for (int g = ni + 1; g <= kk; ++g) {
             const int sb = (cur + g - 1) & 1;
             const uint32_t* S = lane0 + (sb ? (size_t)rows * stride : 0);
-            uint32_t* D = const_cast<uint32_t*>(lane0) + (sb ? 0 : (size_t)rows * stride);
+            uint32_t* D = lane0 + (sb ? 0 : (size_t)rows * stride);
             const int lo = top ? K : K - kk + g, hi = bottom ? K + B : K + B + kk - g;
-            resident_pass<WPL>(S, D, lo, hi, group, 0, j.groups, stride, cm, rag);
+            resident_pass(S, D, lo, hi, group, 0, j.groups, stride, PL, mask, rag);
             __syncthreads();
         }
         cur = (cur + kk) & 1;
         left -= kk;
     }
     // The band after the last generation.
-    if (mine_lane) {
-        const uint32_t* Aw = lane0w + (cur ? (size_t)rows * stride : 0);
+    if (mover) {
+        const uint32_t* A = lane0 + (cur ? (size_t)rows * stride : 0);
         for (int r = group; r < B; r += j.groups) {
-            uint32_t v[WPL];
-            lds_words_gen<WPL>(Aw + (size_t)(K + r) * stride, v);
-            band_store<WPL>(j.dst + (size_t)(y0 + r) * j.pitch + col, gvec, nw, v);
+            uint32_t v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] = A[(size_t)(K + r) * stride + resident_plane(i) * PL];
+            deinterleave4(v);
+            band_store(j.dst + (size_t)(y0 + r) * j.pitch + col, dvec, nw, v);
         }
     }
     return true;
 }
 
 // One grid: CTA c runs band c.
-template <int WPL, int LANES>
+template <int LANES>
 __global__ void __launch_bounds__(kResidentMaxThreads, 1) rows_resident_kernel(ResidentLaunch a) {
     extern __shared__ __align__(16) uint32_t smem[];
     __shared__ int stop;
@@ -416,9 +462,7 @@ __global__ void __launch_bounds__(kResidentMaxThreads, 1) rows_resident_kernel(R
     j.src = a.src;
     j.dst = a.dst;
     j.pub = a.pub;
-    j.done = a.epoch_done;
     j.pitch = a.W;
-    j.ppitch = a.W;
     j.W = a.W;
     j.Y = a.Y;
     j.K = a.K;
@@ -427,31 +471,7 @@ __global__ void __launch_bounds__(kResidentMaxThreads, 1) rows_resident_kernel(R
     j.b = blockIdx.x;
     j.nb = gridDim.x;
     j.gens = a.gens;
-    resident_band<WPL, LANES>(j, smem, &stop, a.status, a.spin_limit);
-}
-
-// Many grids: persistent CTAs (all resident: a cooperative launch) take
-// bands in ticket order and run each to its last generation. The bands of a
-// grid have consecutive tickets, so a band's neighbours are always taken by
-// CTAs that are running or will be as soon as one frees up: a grid has at
-// most as many bands as there are CTAs, and bands of earlier grids never
-// wait on later tickets.
-template <int WPL>
-__global__ void __launch_bounds__(kResidentMaxThreads, 1)
-batch_resident_kernel(const ResidentBand* __restrict__ jobs, int njobs, int* ticket, int* status,
-                      long long spin_limit) {
-    extern __shared__ __align__(16) uint32_t smem[];
-    __shared__ int stop;
-    __shared__ int job;
-    for (;;) {
-        if (threadIdx.x == 0) job = atomicAdd(ticket, 1);
-        __syncthreads();
-        const int t = job;
-        if (t >= njobs) return;
-        const ResidentBand j = jobs[t];
-        if (!resident_band<WPL, 0>(j, smem, &stop, status, spin_limit)) return;
-        __syncthreads();   // shared memory and `job` are reused by the next band
-    }
+    resident_band<LANES>(j, smem, &stop, a.status, a.spin_limit);
 }
 
 } // namespace golb200

@@ -71,9 +71,8 @@ struct RoundBuffers {
     // resident rounds (GOL_SERVE_RESIDENT): bands, exchange slots, counters
     golb200::ResidentBand* d_rjobs = nullptr;
     golb200::ResidentBand* h_rjobs = nullptr;   // pinned staging
-    uint32_t* d_rpub = nullptr;
-    int* d_rdone = nullptr;
-    size_t cap_rjobs = 0, cap_rpub = 0, cap_rdone = 0;
+    unsigned long long* d_rpub = nullptr;
+    size_t cap_rjobs = 0, cap_rpub = 0;
     std::vector<uint64_t> ids;               // request of each grid of the round
     golb200::BatchGrid* h_grids = nullptr;   // pinned staging
     golb200::BatchItem* h_items = nullptr;
@@ -193,7 +192,7 @@ int ensure_round_capacity(gol_server* s, RoundBuffers& r, size_t grids, size_t i
     return GOL_OK;
 }
 
-int ensure_resident_capacity(gol_server* s, RoundBuffers& r, size_t jobs, size_t pub, size_t done) {
+int ensure_resident_capacity(gol_server* s, RoundBuffers& r, size_t jobs, size_t pub) {
     cudaError_t ce = cudaSuccess;
     auto grow = [&](size_t need, size_t& cap, auto** dptr, auto** hptr) {
         if (need <= cap || ce != cudaSuccess) return;
@@ -206,8 +205,7 @@ int ensure_resident_capacity(gol_server* s, RoundBuffers& r, size_t jobs, size_t
         cap = ce == cudaSuccess ? n : 0;
     };
     grow(std::max<size_t>(jobs, 1), r.cap_rjobs, &r.d_rjobs, &r.h_rjobs);
-    grow(std::max<size_t>(pub, 1), r.cap_rpub, &r.d_rpub, static_cast<uint32_t**>(nullptr));
-    grow(std::max<size_t>(done, 1), r.cap_rdone, &r.d_rdone, static_cast<int**>(nullptr));
+    grow(std::max<size_t>(pub, 1), r.cap_rpub, &r.d_rpub, static_cast<unsigned long long**>(nullptr));
     if (ce != cudaSuccess) return s->cuda_fail(ce, "resident round buffers");
     return GOL_OK;
 }
@@ -448,17 +446,17 @@ static int queue_resident_round(gol_server* s, RoundBuffers& rb) {
     s->running.swap(still);
     int rc = ensure_round_capacity(s, rb, grids.size(), 1, 1, 1);
     if (rc) return rc;
-    if ((rc = ensure_resident_capacity(s, rb, (size_t)plan.ndone, plan.pub_words, (size_t)plan.ndone)))
+    if ((rc = ensure_resident_capacity(s, rb, (size_t)plan.nbands, plan.pub_words)))
         return rc;
-    golb200::fill_resident_jobs(plan, grids.data(), rb.d_rpub, rb.d_rdone, rb.h_rjobs);
-    cudaError_t ce = cudaMemcpyAsync(rb.d_rjobs, rb.h_rjobs, (size_t)plan.ndone * sizeof(golb200::ResidentBand),
+    golb200::fill_resident_jobs(plan, grids.data(), rb.d_rpub, rb.h_rjobs);
+    cudaError_t ce = cudaMemcpyAsync(rb.d_rjobs, rb.h_rjobs, (size_t)plan.nbands * sizeof(golb200::ResidentBand),
                                      cudaMemcpyHostToDevice, s->stream);
-    if (ce == cudaSuccess) ce = cudaMemsetAsync(rb.d_rdone, 0, (size_t)std::max(plan.ndone, 1) * sizeof(int), s->stream);
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(rb.d_rpub, 0, std::max<size_t>(plan.pub_words, 1) * sizeof(unsigned long long), s->stream);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(rb.d_ticket, 0, sizeof(int), s->stream);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(rb.d_status, 0, sizeof(int), s->stream);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(rb.d_still, 0, grids.size() * sizeof(int), s->stream);
-    if (ce == cudaSuccess && plan.ndone)
-        ce = golb200::launch_batch_resident(rb.d_rjobs, plan.ndone, rb.d_ticket, rb.d_status, plan, s->stream);
+    if (ce == cudaSuccess && plan.nbands)
+        ce = golb200::launch_batch_resident(rb.d_rjobs, plan.nbands, rb.d_ticket, rb.d_status, plan, s->stream);
     if (ce == cudaSuccess)
         ce = cudaMemcpyAsync(rb.h_status, rb.d_status, sizeof(int), cudaMemcpyDeviceToHost, s->stream);
     if (ce == cudaSuccess)
@@ -825,7 +823,6 @@ void gol_serve_destroy(gol_server* s) {
         if (r.d_rjobs) cudaFree(r.d_rjobs);
         if (r.h_rjobs) cudaFreeHost(r.h_rjobs);
         if (r.d_rpub) cudaFree(r.d_rpub);
-        if (r.d_rdone) cudaFree(r.d_rdone);
         if (r.done_event) cudaEventDestroy(r.done_event);
     }
     if (s->arena) cudaFree(s->arena);
