@@ -5,14 +5,24 @@
 // generation counts advance together:
 //
 //   work item   (grid, x-slice, band group, pass): one pass of k generations
-//               on one warp. Narrow grids (W / WPL <= 32 lanes) have one
-//               slice and cut the warp into S segments of L = W / WPL lanes
-//               (any L, so narrow grids keep most lanes busy), each segment
-//               streaming its own band through the K-stage pipeline
-//               (band_tile's step code in segmented mode). Wider grids are
-//               cut into slices of 30 lanes plus a halo lane each side
-//               (errors from the unknown cells beyond the halo move one cell
-//               per generation and stay in the halo for k <= 32).
+//               on one warp, in the register-block form (block_group below;
+//               gol_rows_block.cuh): rows of more than 30 words in slices of
+//               up to 30 columns with a context lane each side, narrower ones
+//               in segments of W + 1 lanes, a band each. Its one body serves
+//               every depth and band height, so each grid has its own, and an
+//               item of 16 rows and 8 generations takes about 5 us where one
+//               of the pipeline took 9 for 4 generations (serving 24 requests
+//               27.5 -> 15.4 ms, a batch of 48 grids 14.9 -> 12.3 ms, of 512
+//               tracked 75 -> 56 ms).
+//               Grids with a forced lane width run the K-stage pipeline
+//               instead (the whole batch does): narrow grids (W / WPL <= 32
+//               lanes) have one slice and cut the warp into S segments of
+//               L = W / WPL lanes (any L, so narrow grids keep most lanes
+//               busy), each segment streaming its own band (band_tile's step
+//               code in segmented mode). Wider grids are cut into slices of
+//               30 lanes plus a halo lane each side (errors from the unknown
+//               cells beyond the halo move one cell per generation and stay in
+//               the halo for k <= 32).
 //   order       items are numbered critical-path first: by descending
 //               remaining passes of their grid, so the longest grids start
 //               at once and short ones fill in; persistent one-warp CTAs
@@ -29,12 +39,13 @@
 //               unfinished item (a CTA claims tickets in increasing order),
 //               so it is running or about to run that item: the wait always
 //               ends, and the bound is only a guard.
-//   release     each lane fences its stores, the warp syncs, lane 0 stores
-//               the new pass count with st.release.
+//   release     the warp syncs, lane 0 stores the new pass count with
+//               st.release.
 //
-// Rows are read through cp.async after the acquire; a weak load ordered
-// after an acquire observes the released data (PTX memory model), so L1
-// cannot serve a stale line of a buffer rewritten in this same launch.
+// The pipeline reads rows through cp.async after the acquire; a weak load
+// ordered after an acquire observes the released data (PTX memory model), so
+// L1 cannot serve a stale line of a buffer rewritten in this same launch. The
+// register-block form reads them through L2.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -47,6 +58,7 @@
 
 #include "gol_b200.h"
 #include "gol_internal.h"
+#include "gol_rows_block.cuh"
 #include "gol_rows_resident.cuh"
 #include "gol_rows_temporal.cuh"
 
@@ -155,6 +167,40 @@ __device__ __forceinline__ uint32_t seg_group(const BatchGrid& G, int group, int
     return s.diff;
 }
 
+// One work item in the register-block form (gol_rows_block.cuh): rows of more
+// than 30 words in slices of up to 30 columns with a context lane each side,
+// narrower ones in segments of W + 1 lanes, the dead one first. Rows are read
+// through L2 (another CTA of this launch wrote them).
+constexpr int kBatchBlockR = 64;
+
+template <bool TRACK>
+__device__ __forceinline__ uint32_t block_group(int k, const BatchGrid& G, int group, int slice_idx,
+                                                const uint32_t* src, uint32_t* dst) {
+    const int lane = threadIdx.x & 31;
+    const int seg = G.halo ? 0 : lane / G.seg_lanes;
+    const int col = (G.halo ? slice_idx * G.slice + lane : lane - seg * G.seg_lanes) - 1;
+    const int ys = (group * G.segs + seg) * G.band, y0 = ys - k;
+    const bool ok = seg < G.segs && col >= 0 && col < G.W && ys < G.Y;
+    const bool own = ok && (!G.halo || (lane >= 1 && lane <= G.slice));
+    const int n = G.band + 2 * k;
+    const bool inside = __all_sync(0xffffffffu, ok && y0 >= 0 && y0 + block_rows(n) <= G.Y);
+    const int W = G.W, band = G.band, rows = own ? min(G.band, G.Y - ys) : 0;
+    uint32_t w[kBatchBlockR];
+    block_load<kBatchBlockR, true>(w, src + (long long)y0 * W + col, W, inside, ok, y0, G.Y, n);
+    block_generations<kBatchBlockR>(w, band, k, inside, ok, y0, G.Y);
+    const uint32_t* old = src + (long long)ys * W + col;
+    uint32_t* d = dst + (long long)ys * W + col;
+    uint32_t diff = 0u;
+#pragma unroll
+    for (int r = 0; r < kBatchBlockR - 2; ++r, d += W, old += W) {
+        if (r < rows) {
+            if (TRACK) diff |= w[r] ^ __ldcg(old);
+            *d = w[r];
+        }
+    }
+    return diff;
+}
+
 template <int WPL, bool TRACK>
 __device__ __forceinline__ uint32_t seg_dispatch(int k, const BatchGrid& G, int group, int slice,
                                                  const uint32_t* src, uint32_t* dst,
@@ -219,13 +265,14 @@ constexpr int batch_min_blocks() {
                : (WPL_ONLY == 1 ? 19 : WPL_ONLY == 2 ? 15 : GOL_BATCH_MIN_BLOCKS);
 }
 
-template <int WPL_ONLY, bool TRACK>
-__global__ void __launch_bounds__(32, (batch_min_blocks<WPL_ONLY, TRACK>()))
+template <int WPL_ONLY, bool TRACK, bool BLOCK = false>
+__global__ void __launch_bounds__(32, (BLOCK ? 20 : batch_min_blocks<WPL_ONLY, TRACK>()))
 batch_kernel(const BatchGrid* __restrict__ grids, const BatchItem* __restrict__ items, int nitems,
              int* ticket, int* done, int* status, unsigned long long* census, long long spin_limit) {
     // the row ring, and with TRACK the old-row ring right after it
     __shared__ __align__(16) uint32_t
-        ring[kRowRing * 32 * (WPL_ONLY ? WPL_ONLY : 4) * (TRACK && GOL_BATCH_TRACK_OLD == 3 ? 2 : 1)];
+        ring[BLOCK ? 1 : kRowRing * 32 * (WPL_ONLY ? WPL_ONLY : 4) *
+                             (TRACK && GOL_BATCH_TRACK_OLD == 3 ? 2 : 1)];
     constexpr int kEdgeWords = WPL_ONLY == 1 ? 1 : seg_edge_words(kBatchMaxK);   // 1: shuffles
     __shared__ uint32_t etab[kEdgeWords];
     const int lane = threadIdx.x & 31;
@@ -270,29 +317,40 @@ batch_kernel(const BatchGrid* __restrict__ grids, const BatchItem* __restrict__ 
         const int dep = lane < nj * ns ? (jlo + lane / ns) * G.nslices + slo + lane % ns : -1;
         const long long t_wait = clock64();
         if (it.pass > 0) {
-            // Lane d polls dependency d until it reached this pass; then every
-            // lane acquires every counter (each is already there), so each
-            // lane's own copies below are ordered after the producers' releases.
+            // Lane d polls dependency d until it reached this pass. The warp
+            // barrier after the vote orders every lane's reads after all the
+            // acquires; that is enough where rows are read through L2 (the
+            // register-block form). Copies through L1 want an acquire of their
+            // own lane: there every lane acquires every counter (each is
+            // already there), one after the other.
             bool ok = true;
             if (dep >= 0) {
                 const int* p = done + G.done_base + dep;
                 long long spins = 0;
-                while (ld_acquire(p) < it.pass) {
-                    if (++spins > spin_limit || *(volatile int*)status != 0) {
+                // A pass takes microseconds: a warp whose item is passes away
+                // sleeps as many, so that the warps that claimed items far
+                // ahead do not crowd the counters (a lone 2048^2 grid: 14.2 us
+                // a pass with all of them polling).
+                for (int v; (v = ld_acquire(p)) < it.pass;) {
+                    const unsigned ns = it.pass - v > 1 ? 1000u * min(it.pass - v - 1, 64) : 64u;
+                    if ((spins += ns / 64) > spin_limit || *(volatile int*)status != 0) {
                         ok = false;
                         break;
                     }
-                    __nanosleep(64);
+                    __nanosleep(ns);
                 }
             }
             if (!__all_sync(0xffffffffu, ok)) {
                 if (lane == 0) atomicCAS(status, 0, GOL_E_TIMEOUT);
                 return;
             }
-            int seen = 0;
-            for (int d = 0; d < nj * ns; ++d)
-                seen |= ld_acquire(done + G.done_base + (jlo + d / ns) * G.nslices + slo + d % ns);
-            asm volatile("" ::"r"(seen));
+            __syncwarp();
+            if constexpr (!BLOCK) {
+                int seen = 0;
+                for (int d = 0; d < nj * ns; ++d)
+                    seen |= ld_acquire(done + G.done_base + (jlo + d / ns) * G.nslices + slo + d % ns);
+                asm volatile("" ::"r"(seen));
+            }
         }
         // Claim the next item now: the atomic's round trip overlaps the work.
         int next = 0;
@@ -312,7 +370,9 @@ batch_kernel(const BatchGrid* __restrict__ grids, const BatchItem* __restrict__ 
             const uint32_t* src = odd ? G.buf[1] : G.buf[0];
             uint32_t* dst = odd ? G.buf[0] : G.buf[1];
             uint32_t diff;
-            if constexpr (WPL_ONLY != 0) {
+            if constexpr (BLOCK) {
+                diff = block_group<TRACK>(k, G, it.group, it.slice, src, dst);
+            } else if constexpr (WPL_ONLY != 0) {
                 diff = seg_dispatch<WPL_ONLY, TRACK>(k, G, it.group, it.slice, src, dst, ring, etab);
             } else {
                 switch (G.wpl) {
@@ -327,7 +387,8 @@ batch_kernel(const BatchGrid* __restrict__ grids, const BatchItem* __restrict__ 
         uint32_t* trk = TRACK ? ld_ptr_again(&gp->trk) : nullptr;
         if (TRACK && trk && lane == 0)   // this pass's flag, read by the next pass
             *(volatile uint32_t*)(trk + (odd ? nper : 0) + cell) = (changed || k != G.k) ? 1u : 0u;
-        __threadfence();
+        // (the release is cumulative over what the warp barrier orders before it)
+        if constexpr (!BLOCK) __threadfence();
         __syncwarp();
         if (lane == 0) {
             if (TRACK && trk)
@@ -452,6 +513,7 @@ bool choose_batch_plan(int W, int Y, uint64_t gens, int force_wpl, int force_k, 
                 const double score = cost / std::max(parallel, 1.0) + crit_weight * crit;
                 if (!found || score < out->score) {
                     found = true;
+                    out->block = false;
                     out->wpl = wpl;
                     out->k = k;
                     out->band = band;
@@ -469,6 +531,44 @@ bool choose_batch_plan(int W, int Y, uint64_t gens, int force_wpl, int force_k, 
                 }
                 if (force_band) break;
             }
+        }
+    }
+    return found;
+}
+
+// The register-block form. In scheduler cycles, an item of B rows and k
+// generations takes about k (B + k + 1.5) row-generations (the rows shrink by
+// two a generation) at 23.5 cycles beside other warps and 28.5 alone, 12 a
+// row for loads and stores, and 800 for its ticket, dependencies and release;
+// alone, in its grid's chain, about 5000 for their latency and the rows'. Both
+// depths and band heights are a grid's own (one kernel body serves them all).
+bool choose_block_plan(int W, int Y, uint64_t gens, int force_k, int force_band, GridChoice* out,
+                       double parallel, double crit_weight) {
+    bool found = false;
+    const bool sliced = W > kBlockOwn;
+    const int nslices = sliced ? (W + kBlockOwn - 1) / kBlockOwn : 1;
+    const int slice = (W + nslices - 1) / nslices;
+    for (int k : {1, 2, 3, 4, 8}) {
+        if (force_k ? k != force_k : k < 4) continue;
+        for (int band : {8, 12, 16, 24, 32, 40, 48, 56}) {
+            if (force_band) band = force_band;
+            if (band >= k && band + 2 * k <= kBatchBlockR) {
+                const int S = sliced ? 1 : std::max(1, std::min(31 / (W + 1), (Y + band - 1) / band));
+                const int ngroups = (Y + S * band - 1) / (S * band);
+                const uint64_t passes = (gens + k - 1) / k;
+                const double rows = (double)k * (band + k + 1.5);
+                const double cost = (double)passes * nslices * ngroups *
+                                    (rows * 23.5 + 12 * (band + 2 * k) + 800);
+                const double crit = (double)passes * (rows * 28.5 + 5000);
+                const double score = cost / std::max(parallel, 1.0) + crit_weight * crit;
+                if (!found || score < out->score) {
+                    found = true;
+                    *out = {1, k, band, sliced ? 32 : W + 1, S, ngroups, (int)passes,
+                            gens % k ? (int)(gens % k) : k, sliced ? slice : W, nslices,
+                            sliced ? 1 : 0, true, cost, crit, score};
+                }
+            }
+            if (force_band) break;
         }
     }
     return found;
@@ -500,6 +600,15 @@ template <int W, bool TR>
 static int ctas_per_sm_of() {
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel<W, TR>, 32, 0) !=
+        cudaSuccess)
+        per_sm = 1;
+    return std::max(1, per_sm);
+}
+
+template <bool TR>
+static int block_ctas_per_sm() {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel<1, TR, true>, 32, 0) !=
         cudaSuccess)
         per_sm = 1;
     return std::max(1, per_sm);
@@ -547,6 +656,7 @@ void batch_grid_from_choice(const GridChoice& ch, int W, int Y, BatchGrid* g) {
     g->slice = ch.slice;
     g->nslices = ch.nslices;
     g->halo = ch.halo;
+    g->block = ch.block;
 }
 
 template <int W, bool TR>
@@ -560,10 +670,26 @@ static void launch_batch_variant(int ctas, cudaStream_t stream, const BatchGrid*
 cudaError_t launch_batch_kernel(const BatchGrid* d_grids, const BatchItem* d_items, int nitems,
                                 int* d_ticket, int* d_done, int* d_status, int num_sms,
                                 cudaStream_t stream, unsigned long long* d_census, int wpl_only,
-                                long long spin_limit, bool track) {
+                                long long spin_limit, bool track, int block_width) {
     if (spin_limit <= 0) spin_limit = kSpinLimit;
     if (nitems <= 0) return cudaSuccess;
     // every CTA resident at once (the dependency waits rely on it)
+    if (block_width) {
+        // No more warps than a pass of every grid has items (four per SM at
+        // least): those beyond would only wait, and a small grid's items would
+        // land on the same schedulers by chance (a lone 2048^2 grid: 12.0 us a
+        // pass with 20 warps per SM, 9.4 so).
+        static const int fit[2] = {block_ctas_per_sm<false>(), block_ctas_per_sm<true>()};
+        const int per_sm = std::min(fit[track], std::max(4, (block_width + num_sms - 1) / num_sms));
+        const int n = std::min(nitems, num_sms * per_sm);
+        if (track)
+            batch_kernel<1, true, true><<<n, 32, 0, stream>>>(d_grids, d_items, nitems, d_ticket, d_done,
+                                                              d_status, d_census, spin_limit);
+        else
+            batch_kernel<1, false, true><<<n, 32, 0, stream>>>(d_grids, d_items, nitems, d_ticket, d_done,
+                                                               d_status, d_census, spin_limit);
+        return cudaPeekAtLastError();
+    }
     const int ctas = std::min(nitems, num_sms * batch_kernel_ctas_per_sm(wpl_only, track));
 #define GOL_BATCH_ARGS ctas, stream, d_grids, d_items, nitems, d_ticket, d_done, d_status, d_census, \
                        spin_limit
@@ -887,6 +1013,7 @@ struct gol_batch {
     bool track_any = false;
     int nitems = 0, ngroups_total = 0;
     int wpl_only = 0;                     // lane width shared by every grid (0: mixed)
+    bool block = false;                   // every grid in the register-block form
     bool uploaded = false, ran = false;
     cudaGraphExec_t graph = nullptr;
     // Resident runs (gol_batch_run_resident): bands of every grid, their
@@ -1016,7 +1143,8 @@ int gol_batch_plan(const gol_batch* b, int32_t grid_id, uint32_t* lane_words,
     if (!b || grid_id < 0 || grid_id >= (int)b->grids.size()) return GOL_E_INVALID;
     const auto& e = b->grids[grid_id];
     golb200::GridChoice ch = e.choice;   // the uploaded batch's plan
-    if (!b->uploaded &&
+    if (!b->uploaded && (e.force_wpl || !golb200::choose_block_plan(e.W, e.Y, e.gens, e.force_k,
+                                                                    e.force_band, &ch)) &&
         !golb200::choose_batch_plan(e.W, e.Y, e.gens, e.force_wpl, e.force_k, e.force_band, &ch))
         return GOL_E_UNSUPPORTED;
     if (lane_words) *lane_words = ch.wpl;
@@ -1045,7 +1173,32 @@ int gol_batch_upload(gol_batch* b) {
     // about max(total / num_sms, longest chain * warps per SM) SM time.
     double best_est = -1, parallel = 1;
     std::vector<golb200::GridChoice> best;
+    // The register-block form, unless a grid's lane width is forced (or a band
+    // it does not have): each grid its cheapest plan, then those whose chain
+    // would outlast the batch's work a shorter chain.
+    b->block = true;
+    {
+        std::vector<golb200::GridChoice> ch(b->grids.size());
+        parallel = 4.0 * b->num_sms;
+        double work = 0;
+        auto plan = [&](size_t i, double weight) {
+            const auto& e = b->grids[i];
+            return golb200::choose_block_plan(e.W, e.Y, std::max<uint64_t>(e.gens, 1), e.force_k,
+                                              forced_band(e), &ch[i], parallel, weight);
+        };
+        for (size_t i = 0; i < b->grids.size() && b->block; ++i) {
+            b->block = !b->grids[i].force_wpl && plan(i, 0.0);
+            work += b->block && b->grids[i].gens ? ch[i].cost / parallel : 0;
+        }
+        for (size_t i = 0; i < b->grids.size() && b->block; ++i)
+            if (ch[i].crit > work) plan(i, 1.0);
+        if (b->block) {
+            best = std::move(ch);
+            best_est = 0;
+        }
+    }
     for (int wpl : {4, 2, 1}) {
+        if (b->block) break;
         const double wps = golb200::batch_kernel_ctas_per_sm(wpl);
         const double par = (double)b->num_sms * wps;
         for (int k = golb200::kBatchMaxK; k >= 1; --k) {
@@ -1087,7 +1240,7 @@ int gol_batch_upload(gol_batch* b) {
     // A first pass with fewer items than about two per resident warp leaves
     // SMs idle on every pass: halve the tallest bands (not below 16 rows)
     // until it has enough items.
-    for (int round = 0; round < 3; ++round) {
+    for (int round = 0; round < 3 && !b->block; ++round) {
         double first_pass = 0;
         int tallest = 0;
         for (const auto& e : b->grids) {
@@ -1235,7 +1388,8 @@ int gol_batch_run(gol_batch* b) {
         if (ce == cudaSuccess)
             ce = golb200::launch_batch_kernel(b->d_grids, b->d_items, b->nitems, b->d_ticket,
                                               b->d_done, b->d_status, b->num_sms, cs, b->d_census,
-                                              b->wpl_only, 0, b->track_any);
+                                              b->wpl_only, 0, b->track_any,
+                                              b->block ? b->ngroups_total : 0);
         cudaGraph_t g = nullptr;
         cudaError_t ce2 = cudaStreamEndCapture(cs, &g);
         if (ce == cudaSuccess) ce = ce2;

@@ -197,6 +197,8 @@ struct BatchGrid {
     int slice;             // words per x-slice (W when unsliced)
     int nslices;
     int halo;              // halo words each side of a slice (0 when unsliced)
+    int block;             // nonzero: the register-block form (one word per lane; unsliced
+                           // rows take seg_lanes = W + 1 lanes, a dead one first)
     int done_base;         // offset of this grid's (group, slice) counters
     int parity0;           // buffer holding the grid at the start of the launch
     // Change tracking (trk null: every item is computed). An item is a tile:
@@ -225,6 +227,7 @@ constexpr int kBatchMaxK = 4;
 
 struct GridChoice {
     int wpl, k, band, seg_lanes, segs, ngroups, passes, last_k, slice, nslices, halo;
+    bool block;     // the register-block form (choose_block_plan)
     double cost;    // total work
     double crit;    // dependency chain
     double score;   // what the autotuner minimised
@@ -234,6 +237,10 @@ struct GridChoice {
 // Minimises work / parallel + crit_weight * (the grid's dependency chain).
 bool choose_batch_plan(int W, int Y, uint64_t gens, int force_wpl, int force_k, int force_band,
                        GridChoice* out, double parallel = 1.0, double crit_weight = 0.0);
+// The same for the register-block form (any depth up to 8 per grid); costs in
+// scheduler cycles, parallel = schedulers.
+bool choose_block_plan(int W, int Y, uint64_t gens, int force_k, int force_band, GridChoice* out,
+                       double parallel = 1.0, double crit_weight = 0.0);
 
 // Emits the work items of `grids` in critical-path-first order: descending
 // remaining passes (passes - pass), so long grids start first and every
@@ -255,12 +262,14 @@ void batch_grid_from_choice(const GridChoice& ch, int W, int Y, BatchGrid* g);
 // order); done[] and *ticket, *status must be zero. All CTAs fit at once.
 // wpl_only: the lane width all grids share (batch_uniform_wpl), or 0.
 // spin_limit: polls before a dependency wait gives up (0 = the default guard).
-// track: some grid has change tracking (the kernel variant that compares
+// block_width: the items of one pass of every grid where all are in the
+// register-block form, else 0. track: some grid has change tracking (the kernel variant that compares
 // every stored word with its input).
 cudaError_t launch_batch_kernel(const BatchGrid* d_grids, const BatchItem* d_items, int nitems,
                                 int* d_ticket, int* d_done, int* d_status, int num_sms,
                                 cudaStream_t stream, unsigned long long* d_census = nullptr,
-                                int wpl_only = 0, long long spin_limit = 0, bool track = false);
+                                int wpl_only = 0, long long spin_limit = 0, bool track = false,
+                                int block_width = 0);
 
 cudaError_t launch_pack_cells(const uint8_t* cells, uint32_t* words, size_t x, size_t y,
                               cudaStream_t stream);

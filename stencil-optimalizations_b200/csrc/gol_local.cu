@@ -466,6 +466,7 @@ __global__ void __launch_bounds__(32 * kLocalWarps, 5) local_pass_kernel(LocalPa
             if ((ends >> b) & 1u) list[at++] = (uint16_t)(e | kRoleRight);
         }
         __syncthreads();
+        const int tall = a.rows + 2 * a.K;
         for (int w0 = warp * kWindowOwn; w0 < nl; w0 += kLocalWarps * kWindowOwn) {
             // Lanes past either end of the list repeat its first or last
             // entry, and store nothing.
@@ -477,9 +478,9 @@ __global__ void __launch_bounds__(32 * kLocalWarps, 5) local_pass_kernel(LocalPa
                             (role == kRoleLeft ? -1 : role == kRoleRight ? 1 : 0);
             const int y0 = tile_y * a.rows - a.K;
             const bool ok = col >= 0 && col < a.W;
-            const bool inside = __all_sync(0xffffffffu, ok && y0 >= 0 && y0 + R <= a.Y);
+            const bool inside = __all_sync(0xffffffffu, ok && y0 >= 0 && y0 + block_rows(tall) <= a.Y);
             uint32_t w[R];
-            block_load<R>(w, a.src + (long long)y0 * a.W + col, a.W, inside, ok, y0, a.Y);
+            block_load<R>(w, a.src + (long long)y0 * a.W + col, a.W, inside, ok, y0, a.Y, tall);
             block_generations<R>(w, a.rows, a.K, inside, ok, y0, a.Y);
             const bool own = role == kRoleTile && lane >= 1 && lane <= kWindowOwn && g < nl;
             const int rows = min(a.rows, a.Y - tile_y * a.rows);
@@ -501,6 +502,7 @@ __global__ void __launch_bounds__(32 * kLocalWarps, 5) local_pass_kernel(LocalPa
         if (mine) a.cur[t] = flags[threadIdx.x];
     } else {
         const long long line = a.W + 1;
+        const int tall = a.dense_rows + 2 * a.K;
         for (int win = gwarp; win < a.dense_wins; win += nwarps) {
             const long long idx = (long long)win * kBlockOwn - 1 + lane;
             const int block = idx < 0 ? 0 : (int)(idx / line);
@@ -508,9 +510,9 @@ __global__ void __launch_bounds__(32 * kLocalWarps, 5) local_pass_kernel(LocalPa
             const bool ok = idx >= 0 && block < a.dense_blocks && col < a.W;
             const bool own = ok && lane >= 1 && lane <= kBlockOwn;
             const int ys = block * a.dense_rows, y0 = ys - a.K;
-            const bool inside = __all_sync(0xffffffffu, ok && y0 >= 0 && y0 + kDenseR <= a.Y);
+            const bool inside = __all_sync(0xffffffffu, ok && y0 >= 0 && y0 + block_rows(tall) <= a.Y);
             uint32_t w[kDenseR];
-            block_load<kDenseR>(w, a.src + (long long)y0 * a.W + col, a.W, inside, ok, y0, a.Y);
+            block_load<kDenseR>(w, a.src + (long long)y0 * a.W + col, a.W, inside, ok, y0, a.Y, tall);
             block_generations<kDenseR>(w, a.dense_rows, a.K, inside, ok, y0, a.Y);
             // Lanes of one flag word close each tile row together. (The loop
             // below is uniform: it covers the block's full height, rows past

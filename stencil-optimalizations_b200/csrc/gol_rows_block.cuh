@@ -63,19 +63,35 @@ __device__ __forceinline__ void block_hsum(uint32_t c, uint32_t& h0, uint32_t& h
     hsum(lw, c, rw, h0, h1);
 }
 
-// Rows y0 .. y0 + R - 1 of one column into registers (p points at row y0 of
-// it; it is dereferenced inside the grid only). inside: every row and column
-// of the warp lies in the grid; ok: this lane's column does.
-template <int R>
+// Rows that block_load reads for n wanted ones.
+__host__ __device__ constexpr int block_rows(int n) { return (n + 7) & ~7; }
+
+// Rows y0 .. y0 + n - 1 of one column into registers, eight at a time (p
+// points at row y0 of it; it is dereferenced inside the grid only). inside:
+// every row read and every column of the warp lies in the grid; ok: this
+// lane's column does. CG: through L2 only, for rows that other CTAs of the
+// same launch write.
+template <int R, bool CG = false>
 __device__ __forceinline__ void block_load(uint32_t (&w)[R], const uint32_t* p, int pitch,
-                                           bool inside, bool ok, int y0, int Y) {
+                                           bool inside, bool ok, int y0, int Y, int n) {
     if (inside) {
 #pragma unroll
-        for (int r = 0; r < R; ++r, p += pitch) w[r] = __ldg(p);
+        for (int r0 = 0; r0 < R; r0 += 8) {
+            if (r0 < n) {
+#pragma unroll
+                for (int r = r0; r < r0 + 8 && r < R; ++r, p += pitch)
+                    w[r] = CG ? __ldcg(p) : __ldg(p);
+            } else {
+#pragma unroll
+                for (int r = r0; r < r0 + 8 && r < R; ++r) w[r] = 0u;
+            }
+        }
     } else {
 #pragma unroll
-        for (int r = 0; r < R; ++r, p += pitch)
-            w[r] = ok && (unsigned)(y0 + r) < (unsigned)Y ? __ldg(p) : 0u;
+        for (int r = 0; r < R; ++r, p += pitch) {
+            const bool v = r < n && ok && (unsigned)(y0 + r) < (unsigned)Y;
+            w[r] = !v ? 0u : CG ? __ldcg(p) : __ldg(p);
+        }
     }
 }
 
@@ -108,8 +124,12 @@ __device__ __forceinline__ void block_generations(uint32_t (&w)[R], int B, int K
         }
         if (!inside) {   // columns and rows outside the grid stay dead
 #pragma unroll
-            for (int r = 0; r < R; ++r)
-                w[r] = ok && (unsigned)(y0 + g + r) < (unsigned)Y ? w[r] : 0u;
+            for (int r0 = 0; r0 < R; r0 += 8) {
+                if (r0 >= 8 && r0 >= n) break;
+#pragma unroll
+                for (int r = r0; r < r0 + 8 && r < R; ++r)
+                    w[r] = ok && (unsigned)(y0 + g + r) < (unsigned)Y ? w[r] : 0u;
+            }
         }
     }
 }
@@ -123,10 +143,11 @@ __global__ void __launch_bounds__(32, block_min_ctas<R>()) rows_block_kernel(Blo
     const int col = (int)(idx - block * line);   // -1: before the first column, W: a dead column
     const bool ok = idx >= 0 && block < a.nblocks && col < a.W;
     const int y0 = block * a.B - a.K;            // row of w[0]
-    const bool inside = __all_sync(0xffffffffu, ok && y0 >= 0 && y0 + R <= a.Y);
+    const bool inside = __all_sync(0xffffffffu, ok && y0 >= 0 && y0 + block_rows(a.B + 2 * a.K) <= a.Y);
     asm volatile("griddepcontrol.wait;" ::: "memory");
     uint32_t w[R];
-    block_load<R>(w, a.src + (long long)y0 * a.pitch + col, a.pitch, inside, ok, y0, a.Y);
+    block_load<R>(w, a.src + (long long)y0 * a.pitch + col, a.pitch, inside, ok, y0, a.Y,
+                  a.B + 2 * a.K);
     block_generations<R>(w, a.B, a.K, inside, ok, y0, a.Y);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (ok && lane >= 1 && lane <= kBlockOwn) {

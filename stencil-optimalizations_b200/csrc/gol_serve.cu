@@ -372,15 +372,19 @@ int gol_serve_create(gol_server** out, int32_t device, uint64_t arena_bytes, uin
     return GOL_OK;
 }
 
-// Every request runs 2 words per lane (1 for an odd word count) at depth
-// 4 with its own band height, so a round's launch holds one pipeline family
-// (mixed families on one SM compete for the instruction cache). Its slot in
-// the arena: the two grid buffers, two counters (items computed / skipped)
+// Every request runs in the register-block form, whose one kernel body serves
+// every depth and band height (pipelines of several widths in one launch
+// compete for the instruction cache). A round lasts as long as its longest
+// request's chain of passes, so the plan weighs the chain beside the work. A
+// request found still is done at once only where its depth divides its
+// generations, so one that 4 divides and 8 does not takes depth 4.
+// Its slot in the arena: the two grid buffers, two counters (items computed / skipped)
 // and, when it tracks changes, its change flags and still pass (the
 // batch kernel's tracking region), kept for the request's whole life.
 static bool plan_request(gol_server* s, Request& r, uint64_t generations) {
-    if (!golb200::choose_batch_plan(r.W, r.Y, std::max<uint64_t>(generations, 1), r.W % 2 ? 1 : 2,
-                                    golb200::kBatchMaxK, 0, &r.plan))
+    if (!golb200::choose_block_plan(r.W, r.Y, std::max<uint64_t>(generations, 1),
+                                    generations % 8 == 4 ? 4 : 0, 0, &r.plan,
+                                    4.0 * s->num_sms, 1.0))
         return false;
     const uint64_t passes = (generations + r.plan.k - 1) / r.plan.k;
     r.tracked = s->track_mode == GOL_TRACK_ON ||
@@ -653,8 +657,7 @@ int gol_serve_step(gol_server* s) {
     if (ce == cudaSuccess)
         ce = golb200::launch_batch_kernel(rb.d_grids, rb.d_items, (int)nitems, rb.d_ticket, rb.d_done,
                                           rb.d_status, s->num_sms, s->stream, s->d_census,
-                                          golb200::batch_uniform_wpl(grids.data(), grids.size()), 0,
-                                          track_any);
+                                          1, 0, track_any, std::max(done, 1));
     if (ce == cudaSuccess)
         ce = cudaMemcpyAsync(rb.h_status, rb.d_status, sizeof(int), cudaMemcpyDeviceToHost, s->stream);
     if (ce == cudaSuccess)
