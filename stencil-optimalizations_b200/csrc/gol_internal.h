@@ -27,6 +27,7 @@ struct RowsPlan {
                            // per thread, nslices = CTAs across the row, no halo
     int block = 0;         // register-block kernel (gol_rows_block.cuh): R, the rows a warp
                            // holds; band = rows it stores, nbands = blocks of rows
+    bool pair = false;     // row-pair pipeline (gol_rows_pair.cuh): band even
 };
 
 // Picks words-per-lane and CTA shape for a W-word by Y-row grid and depth k.
@@ -111,10 +112,16 @@ cudaError_t launch_resident(const uint32_t* src, uint32_t* dst, int W, int Y, lo
                             const ResidentPlan& p, unsigned long long* pub, int* status,
                             cudaStream_t stream, long long spin_limit = 0);
 
+// Row-pair passes can run on grids interleaved by four (interleaved below),
+// which launch_interleave does in place (back: undoes). Rows of whole lanes
+// (W % 4 == 0) without padding, 16-byte aligned.
+cudaError_t launch_interleave(uint32_t* grid, int W, int Y, bool back, cudaStream_t stream);
+
 // One pass of k generations (1 <= k <= kMaxKForWpl(plan.wpl)). pitch: words
 // from one row to the next (0 = W).
 cudaError_t launch_rows_pass(const uint32_t* src, uint32_t* dst, int W, int Y, int k,
-                             const RowsPlan& plan, cudaStream_t stream, int pitch = 0);
+                             const RowsPlan& plan, cudaStream_t stream, int pitch = 0,
+                             bool interleaved = false);
 
 // Change-tracking tiles (GOL_ALG_LOCAL): tile = x-slice x row band.
 struct LocalPlan {

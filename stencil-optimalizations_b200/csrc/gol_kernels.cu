@@ -6,6 +6,7 @@
 #include "gol_b200.h"
 #include "gol_internal.h"
 #include "gol_rows_block.cuh"
+#include "gol_rows_pair.cuh"
 #include "gol_rows_resident.cuh"
 #include "gol_rows_stream.cuh"
 #include "gol_rows_temporal.cuh"
@@ -86,6 +87,26 @@ cudaError_t launch_block(const BlockLaunch& a, cudaStream_t stream) {
     return cudaLaunchKernelEx(&cfg, rows_block_kernel<R>, a);
 }
 
+// The row-pair pipeline, a programmatic dependent too.
+template <bool INTER>
+cudaError_t launch_pair(const RowsLaunch& a, const RowsPlan& p, cudaStream_t stream) {
+    static const cudaError_t attr_ok =
+        cudaFuncSetAttribute(rows_pair_kernel<kPairK, INTER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)pair_smem_bytes(kPairK));
+    if (attr_ok != cudaSuccess) return attr_ok;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(p.nbands, p.nslices);
+    cfg.blockDim = dim3(p.threads);
+    cfg.dynamicSmemBytes = pair_smem_bytes(kPairK);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, rows_pair_kernel<kPairK, INTER>, a);
+}
+
 // Estimated time (us) of a register-block pass and its best block. Fitted to
 // passes at 256^2 .. 16384^2, K = 4 and 8, to about 10 %: a warp takes
 // `rows` row-generations (plus about 2.5 a generation for the exits every
@@ -134,9 +155,55 @@ int device_sm_count(int device) {
     return n > 0 ? n : 148;
 }
 
+// Plans the row-pair pipeline and estimates a pass on interleaved rows (us; 0
+// where rows are not whole lanes): whole waves of CTAs (two of up to four
+// warps per SM, or one), each taking its rows and the K that fill its stages
+// at 0.42 us per two rows and warp on the fullest scheduler, 0.57 for a warp
+// alone there. Against 16384^2 (25.4 us), 12288^2 (20.5), 32768^2 (89) and
+// 8192 x 16384 (18.3) it is 1, -1, 9 and 0 % off.
+static double plan_pair(int W, int Y, int num_sms, RowsPlan* p) {
+    if (W % 4 || W <= 0) return 0;
+    const int lanes = W / 4;
+    int slice = lanes, nslices = 1, halo = 0;
+    if (lanes > kTemporalMaxThreads) {
+        const int per = kTemporalMaxThreads - 2;   // one halo lane each side
+        nslices = (lanes + per - 1) / per;
+        slice = (lanes + nslices - 1) / nslices;
+        nslices = (lanes + slice - 1) / slice;
+        halo = 4;
+    }
+    const int threads = (slice + (halo ? 2 : 0) + 31) / 32 * 32;
+    const int per_sm = threads <= 128 ? 2 : 1;
+    const int target = std::max(1, per_sm * num_sms / nslices);   // CTAs along y per wave
+    double best = 0;
+    const int warps = (per_sm * threads / 32 + 3) / 4;   // per scheduler
+    for (int waves = 1;; ++waves) {   // the fewest waves of bands of up to 120 rows (taller
+                                      // ones leave a long tail: 32768^2 102 us at 222, 89 at 112)
+        int band = (int)(((long long)Y + (long long)target * waves - 1) / ((long long)target * waves));
+        band = std::max(8, (band + 1) / 2 * 2);
+        if (band > 120) continue;
+        best = 1.0 + waves * 0.5 * (band + kPairK) * (warps == 1 ? 0.57 : 0.42 * warps);
+        p->wpl = 4;
+        p->threads = threads;
+        p->band = band;
+        p->nbands = (Y + band - 1) / band;
+        p->slice = slice * 4;
+        p->nslices = nslices;
+        p->halo = halo;
+        break;
+    }
+    p->stream = false;
+    p->block = 0;
+    p->pair = true;
+    return best;
+}
+
+// The depth at which a generation costs least, a tie going to the row-pair
+// pipeline (its interleaved passes against the register-block ones).
 int best_depth(int W, int Y, int num_sms) {
     int best = 4;
     double t = 0;
+    RowsPlan pair;
     for (int k : {4, 6, 8, 12, 16}) {
         const double u = best_block(W, std::max(Y, 1), k, num_sms).us / k;
         if (t == 0 || u < t) {
@@ -144,7 +211,8 @@ int best_depth(int W, int Y, int num_sms) {
             best = k;
         }
     }
-    return best;
+    const double u = plan_pair(W, Y, num_sms, &pair) / kPairK;
+    return u > 0 && u <= t ? kPairK : best;
 }
 
 bool plan_rows(int W, int Y, int k, int band_rows, int wpl, int num_sms, RowsPlan* plan,
@@ -167,8 +235,14 @@ bool plan_rows(int W, int Y, int k, int band_rows, int wpl, int num_sms, RowsPla
     const int lanes = W / wpl;
     plan->stream = k == 1 && !k_stage;
     plan->block = 0;
+    plan->pair = false;
     if (k > 1 && !k_stage && !forced) {
         const BlockChoice c = best_block(W, std::max(Y, 1), k, num_sms);
+        if (k == kPairK) {   // rows as they are take the pipeline an eighth longer
+            const double us = 1.13 * plan_pair(W, Y, num_sms, plan);
+            if (us > 0 && us <= c.us) return true;
+            plan->pair = false;
+        }
         plan->wpl = 1;
         plan->threads = 32;
         plan->block = c.R;
@@ -311,7 +385,7 @@ cudaError_t launch_resident(const uint32_t* src, uint32_t* dst, int W, int Y, lo
 }
 
 cudaError_t launch_rows_pass(const uint32_t* src, uint32_t* dst, int W, int Y, int k,
-                             const RowsPlan& p, cudaStream_t stream, int pitch) {
+                             const RowsPlan& p, cudaStream_t stream, int pitch, bool interleaved) {
     if (Y <= 0 || W <= 0) return cudaSuccess;
     if (p.block) {
         if (k < 1 || p.band + 2 * k > p.block) return cudaErrorInvalidValue;
@@ -325,6 +399,11 @@ cudaError_t launch_rows_pass(const uint32_t* src, uint32_t* dst, int W, int Y, i
         }
     }
     RowsLaunch a{src, dst, W, Y, p.band, p.slice, p.halo, pitch ? pitch : W};
+    if (p.pair) {
+        if (k != kPairK || a.pitch % 4) return cudaErrorInvalidValue;
+        return interleaved ? launch_pair<true>(a, p, stream) : launch_pair<false>(a, p, stream);
+    }
+    if (interleaved) return cudaErrorInvalidValue;
     if (p.stream) {
         if (k != 1) return cudaErrorInvalidValue;
         switch (p.wpl) {
@@ -340,6 +419,23 @@ cudaError_t launch_rows_pass(const uint32_t* src, uint32_t* dst, int W, int Y, i
         case 1: return dispatch_k<1, 1>(k, a, p, stream);
         default: return cudaErrorInvalidValue;
     }
+}
+
+cudaError_t launch_interleave(uint32_t* grid, int W, int Y, bool back, cudaStream_t stream) {
+    const size_t n = (size_t)W / 4 * Y;
+    if (n == 0) return cudaSuccess;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)std::min<size_t>((n + 255) / 256, 148 * 16));
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    auto* g = reinterpret_cast<uint4*>(grid);
+    return back ? cudaLaunchKernelEx(&cfg, interleave_kernel<true>, g, n)
+                : cudaLaunchKernelEx(&cfg, interleave_kernel<false>, g, n);
 }
 
 // ---------------------------------------------------------------------------
