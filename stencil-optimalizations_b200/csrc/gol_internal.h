@@ -27,6 +27,7 @@ struct RowsPlan {
                            // per thread, nslices = CTAs across the row, no halo
     int block = 0;         // register-block kernel (gol_rows_block.cuh): R, the rows a warp
                            // holds; band = rows it stores, nbands = blocks of rows
+    bool once = false;     // with stream: bands loaded whole (rows_once_kernel)
     bool pair = false;     // row-pair pipeline (gol_rows_pair.cuh): band even
 };
 

@@ -15,12 +15,6 @@
 #ifndef GOL_STREAM_THREADS
 #define GOL_STREAM_THREADS 128   // CTA size of the one-generation streaming kernel
 #endif
-#ifndef GOL_STREAM_CTAS_PER_SM
-// Default band of the streaming kernel: about this many CTAs per SM per pass
-// (at 32768^2: 9-row bands; 8-, 12- and 16-row bands ran at 5.40, 5.31 and
-// 5.15 TB/s algorithmic).
-#define GOL_STREAM_CTAS_PER_SM 48
-#endif
 
 namespace golb200 {
 
@@ -67,7 +61,7 @@ cudaError_t launch_stream(const RowsLaunch& a, const RowsPlan& p, cudaStream_t s
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, rows_stream_kernel<WPL>, a);
+    return cudaLaunchKernelEx(&cfg, p.once ? rows_once_kernel<WPL> : rows_stream_kernel<WPL>, a);
 }
 
 // The register-block kernel, a programmatic dependent too.
@@ -254,21 +248,15 @@ bool plan_rows(int W, int Y, int k, int band_rows, int wpl, int num_sms, RowsPla
         return true;
     }
     if (plan->stream) {
-        // One generation: lanes of wpl words across the row in CTAs of up to
-        // GOL_STREAM_THREADS threads, each thread walking `band` rows. The
-        // default band gives about GOL_STREAM_CTAS_PER_SM CTAs per SM (many
-        // waves of short-lived CTAs), never below 8 rows (each band re-reads
-        // one halo row above and one below, from L2) nor above 64.
-        plan->threads = std::min(GOL_STREAM_THREADS, (lanes + 31) / 32 * 32);
+        // One generation: lanes of wpl words across the row, each thread
+        // loading its short band whole, or with a forced band walking that.
+        plan->once = band_rows <= 0;
+        plan->threads = std::min(plan->once ? kOnceThreads : GOL_STREAM_THREADS, (lanes + 31) / 32 * 32);
         plan->nslices = (lanes + plan->threads - 1) / plan->threads;
         plan->slice = plan->threads * wpl;
         plan->halo = 0;
-        int band = band_rows;
-        if (band <= 0) {
-            const long long ctas = (long long)GOL_STREAM_CTAS_PER_SM * num_sms;
-            band = (int)std::min<long long>(64, std::max<long long>(8, ((long long)Y * plan->nslices + ctas - 1) / ctas));
-        }
-        band = std::min(band, std::max(Y, 1));
+        const int band = plan->once ? wpl == 4 ? once_rows<4>() : wpl == 2 ? once_rows<2>() : once_rows<1>()
+                                    : std::min(band_rows, std::max(Y, 1));
         plan->band = band;
         plan->nbands = (Y + band - 1) / band;
         return true;

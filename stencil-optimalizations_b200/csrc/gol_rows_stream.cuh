@@ -175,4 +175,78 @@ rows_stream_kernel(RowsLaunch a) {
                                     h0, h1);
 }
 
+// The same pass with a band short enough to be loaded whole: a thread issues
+// the loads of all its B + 2 rows (and lanes 0 and 31 those of their outer
+// words) before the first is used, then forms the rows two at a time
+// (pair_sum, next_word_pair: ten operations a word, where the walk above takes
+// twelve). This is the form of a pass without a forced band; CTAs as above.
+// Bound by HBM: 32768^2 takes 43.1 us (6.2 TB/s of grid read and written, 95 %
+// of a plain copy) where the walk took 48.8, 16384^2 9.3 against 12.3. Bands of
+// 6 / 8 / 12 / 16 rows in CTAs of 128 ran 32768^2 in 46.1 / 44.1 / 43.4 / 43.8 us,
+// 16 rows in CTAs of 64 in 43.1.
+constexpr int kOnceThreads = 64;
+template <int WPL>
+__host__ __device__ constexpr int once_rows() { return WPL == 4 ? 16 : WPL == 2 ? 16 : 30; }
+
+template <int WPL>
+__global__ void __launch_bounds__(kOnceThreads) rows_once_kernel(RowsLaunch a) {
+    constexpr int B = once_rows<WPL>(), R = B + 2;
+    static_assert(B % 2 == 0, "rows are formed two at a time");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int lane = threadIdx.x & 31;
+    const int nslices = (a.W + a.slice - 1) / a.slice;
+    const int slice = (int)(blockIdx.x % (unsigned)nslices);
+    const int y0 = (int)(blockIdx.x / (unsigned)nslices) * B - 1;   // grid row of read-row 0
+    const int base = slice * a.slice + (int)threadIdx.x * WPL;
+    const bool ok = base < a.W;   // W % WPL == 0: a lane is wholly inside or outside
+    // lane 0's word on the left, lane 31's on the right
+    const int outer = lane == 0 ? -1 : WPL;
+    const bool edge = ok && (lane == 0 ? base > 0 : lane == 31 && base + WPL < a.W);
+    const uint32_t* p = a.src + (long long)y0 * a.pitch + base;   // dereferenced inside the grid only
+    uint32_t v[R][WPL], e[R];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (y0 >= 0 && y0 + R <= a.Y) {
+#pragma unroll
+        for (int r = 0; r < R; ++r, p += a.pitch) {
+            stream_load<WPL>(p, ok, v[r]);
+            e[r] = edge ? __ldg(p + outer) : 0u;
+        }
+    } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r, p += a.pitch) {
+            const bool in = (unsigned)(y0 + r) < (unsigned)a.Y;
+            stream_load<WPL>(p, ok && in, v[r]);
+            e[r] = edge && in ? __ldg(p + outer) : 0u;
+        }
+    }
+    uint32_t h0[4][WPL], h1[4][WPL];   // horizontal sums by read-row mod 4
+    auto sums = [&](int r) {
+        uint32_t lw = __shfl_up_sync(0xffffffffu, v[r][WPL - 1], 1);
+        uint32_t rw = __shfl_down_sync(0xffffffffu, v[r][0], 1);
+        lw = lane == 0 ? e[r] : lw;
+        rw = lane == 31 ? e[r] : rw;
+#pragma unroll
+        for (int w = 0; w < WPL; ++w)
+            hsum(w == 0 ? lw : v[r][w - 1], v[r][w], w == WPL - 1 ? rw : v[r][w + 1], h0[r & 3][w],
+                 h1[r & 3][w]);
+    };
+    sums(0);
+    sums(1);
+    uint32_t* d = a.dst + (long long)(y0 + 1) * a.pitch + base;
+#pragma unroll
+    for (int r = 2; r < R; r += 2, d += 2 * (long long)a.pitch) {   // read-rows r - 1 and r
+        sums(r);
+        sums(r + 1);
+        uint32_t up[WPL], down[WPL];
+#pragma unroll
+        for (int w = 0; w < WPL; ++w) {
+            const PairSum s = pair_sum(h0[(r - 1) & 3][w], h1[(r - 1) & 3][w], h0[r & 3][w], h1[r & 3][w]);
+            up[w] = next_word_pair(h0[(r - 2) & 3][w], h1[(r - 2) & 3][w], s, v[r - 1][w]);
+            down[w] = next_word_pair(h0[(r + 1) & 3][w], h1[(r + 1) & 3][w], s, v[r][w]);
+        }
+        if (ok && y0 + r - 1 < a.Y) store_words<WPL>(d, up);
+        if (ok && y0 + r < a.Y) store_words<WPL>(d + a.pitch, down);
+    }
+}
+
 } // namespace golb200
