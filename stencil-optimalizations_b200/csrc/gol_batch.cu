@@ -1024,6 +1024,8 @@ struct gol_batch {
     int rjobs = 0, rctas = 0;
     size_t rsmem = 0;
     golb200::ResidentBatchPlan rplan;
+    uint32_t* h_stage = nullptr;          // pinned: the grid a fetch brings in (the largest so far)
+    size_t stage_words = 0;
     double last_ms = 0;
     std::string err;
 
@@ -1324,9 +1326,13 @@ int gol_batch_upload(gol_batch* b) {
             hg[gi].pstat = b->d_pstat + e.pstat_offset;
         }
         if (e.W == 0 || e.Y == 0) continue;
-        ce = cudaMemcpy2DAsync(hg[gi].buf[0], (size_t)e.pitch * sizeof(uint32_t), e.words.data(),
-                               (size_t)e.W * sizeof(uint32_t), (size_t)e.W * sizeof(uint32_t), e.Y,
-                               cudaMemcpyHostToDevice, b->stream);
+        if (e.pitch == e.W)
+            ce = cudaMemcpyAsync(hg[gi].buf[0], e.words.data(), e.words.size() * sizeof(uint32_t),
+                                 cudaMemcpyHostToDevice, b->stream);
+        else
+            ce = cudaMemcpy2DAsync(hg[gi].buf[0], (size_t)e.pitch * sizeof(uint32_t), e.words.data(),
+                                   (size_t)e.W * sizeof(uint32_t), (size_t)e.W * sizeof(uint32_t), e.Y,
+                                   cudaMemcpyHostToDevice, b->stream);
     }
     if (ce == cudaSuccess && words)
         ce = cudaMemcpyAsync(b->arena + 2 * words, b->arena, words * sizeof(uint32_t),
@@ -1512,16 +1518,35 @@ int gol_batch_fetch(gol_batch* b, int32_t grid_id, uint8_t* cells) {
     if (!b->uploaded) return b->fail(GOL_E_STATE, "fetch before run");
     auto& e = b->grids[grid_id];
     const int which = e.result_buf;
-    std::vector<uint32_t> words((size_t)e.W * e.Y);
+    const size_t n = (size_t)e.W * e.Y;
+    // Through a pinned buffer (a copy to pageable memory goes through the CUDA
+    // driver's own, a piece at a time); pageable where none can be had.
+    std::vector<uint32_t> pageable;
+    if (n > b->stage_words) {
+        if (b->h_stage) cudaFreeHost(b->h_stage);
+        b->h_stage = nullptr;
+        b->stage_words = 0;
+        if (cudaMallocHost(reinterpret_cast<void**>(&b->h_stage), n * sizeof(uint32_t)) == cudaSuccess)
+            b->stage_words = n;
+        else
+            cudaGetLastError();
+    }
+    uint32_t* words = b->h_stage;
+    if (n > b->stage_words) {
+        pageable.resize(n);
+        words = pageable.data();
+    }
     cudaError_t ce = cudaSuccess;
-    if (!words.empty())
-        ce = cudaMemcpy2DAsync(words.data(), (size_t)e.W * sizeof(uint32_t),
-                               b->arena + e.offset + (size_t)which * e.stride,
+    const uint32_t* from = b->arena + e.offset + (size_t)which * e.stride;
+    if (n && e.pitch == e.W)
+        ce = cudaMemcpyAsync(words, from, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, b->stream);
+    else if (n)
+        ce = cudaMemcpy2DAsync(words, (size_t)e.W * sizeof(uint32_t), from,
                                (size_t)e.pitch * sizeof(uint32_t), (size_t)e.W * sizeof(uint32_t),
                                e.Y, cudaMemcpyDeviceToHost, b->stream);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(b->stream);
     if (ce != cudaSuccess) return b->cuda_fail(ce, "batch fetch");
-    golb200::host_unpack_u8(words.data(), e.x, e.y, cells);
+    golb200::host_unpack_u8(words, e.x, e.y, cells);
     return GOL_OK;
 }
 
@@ -1685,6 +1710,7 @@ void gol_batch_destroy(gol_batch* b) {
     if (!b) return;
     if (b->stream) cudaStreamSynchronize(b->stream);
     batch_free_device(b);
+    if (b->h_stage) cudaFreeHost(b->h_stage);
     if (b->own_stream && b->stream) cudaStreamDestroy(b->stream);
     delete b;
 }

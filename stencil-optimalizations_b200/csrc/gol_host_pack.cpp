@@ -179,6 +179,15 @@ void parallel_rows(size_t y, size_t bytes_per_row, F&& body) {
 
 } // namespace
 
+void host_copy(void* dst, const void* src, size_t bytes) {
+    // by pages, so that the ranges' first touches of dst are spread too
+    constexpr size_t kPage = 4096;
+    parallel_rows((bytes + kPage - 1) / kPage, kPage, [=](size_t p0, size_t p1) {
+        const size_t a = p0 * kPage, b = std::min(bytes, p1 * kPage);
+        std::memcpy(static_cast<char*>(dst) + a, static_cast<const char*>(src) + a, b - a);
+    });
+}
+
 void host_pack_u8(const uint8_t* cells, size_t x, size_t y, uint32_t* words) {
     const size_t W = x / 32;
 #ifdef GOL_HAVE_AVX2_PATH

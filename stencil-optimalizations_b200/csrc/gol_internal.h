@@ -290,6 +290,8 @@ cudaError_t launch_unpack_cells(const uint32_t* words, uint8_t* cells, size_t x,
                                 cudaStream_t stream);
 
 // Host packing between a cell grid and 32-bit row words (multi-threaded).
+// Copies on all host threads (as the packing below).
+void host_copy(void* dst, const void* src, size_t bytes);
 void host_pack_u8(const uint8_t* cells, size_t x, size_t y, uint32_t* words);
 void host_pack_i32(const int32_t* cells, size_t x, size_t y, uint32_t* words);
 void host_unpack_u8(const uint32_t* words, size_t x, size_t y, uint8_t* cells);
