@@ -263,13 +263,15 @@ int gol_local_stats(gol_engine* e, uint64_t* passes, uint64_t* tiles_per_pass,
 /* --- Stateless device entry points -------------------------------------- */
 
 /* One pass of k generations, d_src -> d_dst (device row grids, x/32 words
- * per row, 16-byte aligned, must not overlap). k in 1..16. k = 1 runs the
- * HBM-streaming one-generation kernel (band_rows: rows each thread walks),
- * k >= 2 the K-stage row-band kernel (band_rows: output rows per CTA);
- * band_rows = 0 picks a default. Asynchronous on `stream`. */
+ * per row, 16-byte aligned, must not overlap). k in 1..16. band_rows = 0
+ * picks the kernel and its block by the grid's size and k; a forced
+ * band_rows runs, for k = 1, the HBM-streaming kernel (rows each thread
+ * walks), for k >= 2 the K-stage row-band kernel (output rows per CTA).
+ * Asynchronous on `stream`. */
 int gol_rows_pass(const void* d_src, void* d_dst, uint64_t x, uint64_t y, uint32_t k,
                   uint32_t band_rows, void* stream);
-/* Same with the lane width forced (lane_words 1, 2 or 4; 0 = auto). */
+/* Same with the lane width forced (lane_words 1, 2 or 4; 0 = auto; k >= 2
+ * then runs the K-stage kernel). */
 int gol_rows_pass_ex(const void* d_src, void* d_dst, uint64_t x, uint64_t y, uint32_t k,
                      uint32_t band_rows, uint32_t lane_words, void* stream);
 
@@ -327,10 +329,10 @@ int gol_probe_int_peak(double* lane_ops_per_s, void* stream);
 
 /* Many independent grids, each with its own size and generation count,
  * advanced together by one persistent kernel launch (captured as a CUDA
- * graph). An autotuner picks one words-per-lane width and temporal depth for
- * the whole batch (one pipeline body per launch) and a band height per grid;
- * gol_batch_set_plan overrides a grid's plan (mixed widths then run the
- * general kernel). gol_batch_plan reports the plan of the uploaded batch, or
+ * graph). An autotuner picks a temporal depth (up to 8) and a band height per
+ * grid; gol_batch_set_plan overrides a grid's plan (a forced lane width runs
+ * the whole batch as K-stage pipelines of one width and depth where it can,
+ * mixed widths in the general kernel). gol_batch_plan reports the plan of the uploaded batch, or
  * the grid's own best plan before gol_batch_upload. No reference
  * counterpart: the reference runs one grid per invocation
  * (experiment_manager.hpp:365-394). */
