@@ -488,13 +488,9 @@ __global__ void __launch_bounds__(32 * kLocalWarps, 5) local_pass_kernel(LocalPa
             uint32_t* out = a.dst + (long long)tile_y * a.rows * a.W + col;
             uint32_t diff = 0u;
             if (own) {
-#pragma unroll
-                for (int r = 0; r < R - 2; ++r, old += a.W, out += a.W) {
-                    if (r < rows) {
-                        diff |= w[r] ^ __ldg(old);
-                        *out = w[r];
-                    }
-                }
+                block_store_tracked<R>(
+                    w, rows, old, out, a.W, [](const uint32_t* p) { return __ldg(p); },
+                    [&](int, uint32_t x) { diff |= x; });
                 if (diff) atomicOr(flags + owner, 1u << bit);
             }
         }
@@ -524,13 +520,9 @@ __global__ void __launch_bounds__(32 * kLocalWarps, 5) local_pass_kernel(LocalPa
             uint32_t* out = a.dst + (long long)ys * a.W + col;
             const int rows = own ? min(a.dense_rows, a.Y - ys) : 0;
             unsigned long long changed = 0ull;   // bit r: row r of the block differs
-#pragma unroll
-            for (int r = 0; r < kDenseR - 2; ++r, old += a.W, out += a.W) {
-                if (r < rows) {
-                    if (w[r] != __ldg(old)) changed |= 1ull << r;
-                    *out = w[r];
-                }
-            }
+            block_store_tracked<kDenseR>(
+                w, rows, old, out, a.W, [](const uint32_t* p) { return __ldg(p); },
+                [&](int r, uint32_t x) { if (x) changed |= 1ull << r; });
             for (int r = 0; r < a.dense_rows; r += a.rows, word += a.cw) {
                 const bool diff = (changed >> r & ((1ull << a.rows) - 1ull)) != 0ull;
                 const uint32_t bits = __reduce_or_sync(group, diff ? 1u << (col & 31) : 0u);
