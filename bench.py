@@ -908,7 +908,7 @@ def run_ours(args, d: Dist) -> None:
                 "ops_per_cell_update": ALG_INT_OPS_PER_CELL,
                 "note": "algorithmic ops = the reference full adder's 33 word-ops per 64 cells"}
     # One generation per pass is HBM-bound; deeper passes are bound by the
-    # integer (ALU) pipe (ncu: ALU 84 %, DRAM 12 % at k = 4).
+    # integer (ALU) pipe.
     primary, secondary = (hbm_view, int_view) if best_k == 1 else (int_view, hbm_view)
     roofline = dict(primary)
     roofline.update({"traffic": ncu_traffic(kernel, size), "kernel": kernel,

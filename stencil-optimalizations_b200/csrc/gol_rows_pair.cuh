@@ -22,7 +22,7 @@
 // takes 236 registers; held to 168 or 128 it spills: 33 and 25 T). 16384^2,
 // K = 4, 56-row bands: 25.4 us a pass interleaved (42.4 T cell-updates/s), 28.7
 // as rows are, against 31.4 for the K-stage kernel of gol_rows_temporal.cuh and
-// 33.5 for the register-block kernel at this depth (58 at depth 8); at depths
+// 33.5 for the register-block kernel at this depth (63 at depth 8); at depths
 // 3, 5 and 6 40, 41 and 35 T. It wants bands of about 40 rows or more, since
 // 4 K rows' worth of steps fill and drain the stages.
 #pragma once

@@ -36,7 +36,7 @@
 // cell 4i + j. The cells left and right of a word's are then the words before
 // and after it, and only the outer two neighbours of a lane's four words take
 // a shift: 8.5 operations a word and generation, against 12 for rows as they
-// are, one at a time (9.4 -> 6.5 ms for 8192^2, 4096 generations). A band is
+// are, one at a time (9.4 -> 7.6 ms for 8192^2, 4096 generations). A band is
 // interleaved when it is loaded and restored when it is stored, some 8
 // operations a word each way; the exchange slots hold interleaved rows. The
 // four words are kept in planes (word j of all lanes in a run), so every
