@@ -217,6 +217,8 @@ int best_depth(int W, int Y, int num_sms) {
     return u > 0 && u <= t ? kPairK : best;
 }
 
+constexpr long long kStageWords = 16 << 20;   // 64 MiB a buffer
+
 bool plan_rows(int W, int Y, int k, int band_rows, int wpl, int num_sms, RowsPlan* plan,
                bool k_stage) {
     if (k < 1 || k > kMaxTemporalSteps || W <= 0) return false;
@@ -238,7 +240,19 @@ bool plan_rows(int W, int Y, int k, int band_rows, int wpl, int num_sms, RowsPla
     plan->stream = k == 1 && !k_stage;
     plan->block = 0;
     plan->pair = false;
-    if (k > 1 && !k_stage && !forced) {
+    // Grids whose two buffers fill L2 or more, in one slice of whole warps: the
+    // K-stage pipeline reads each row about once, the blocks of 30 columns
+    // their halos again. Pipeline against the other kernels, us a pass:
+    // 32768^2 64 / 75 and 88 / 96 (k = 2, 3), 16384 x 65536 68 / 78 (k = 2, but
+    // 119 / 102 at k = 3), 24576^2 45 / 45 and 63 / 59, 8192 x 65536 57 / 72 at
+    // k = 4 and 48 / 46 at k = 2; in several slices 65536 x 16384 88 / 73, and
+    // in L2 16384^2 25 / 20.
+    const int lanes4 = W / 4;
+    const bool stages = wpl == 4 && (long long)W * Y >= kStageWords && lanes4 % 32 == 0 &&
+                        lanes4 <= kTemporalMaxThreads &&
+                        ((k == 2 && lanes4 >= 128) || (k == 3 && lanes4 > 224) ||
+                         (k == kPairK && lanes4 <= 64));
+    if (k > 1 && !k_stage && !forced && !stages) {
         const BlockChoice c = best_block(W, std::max(Y, 1), k, num_sms);
         if (k == kPairK) {   // rows as they are take the pipeline an eighth longer
             const double us = 1.13 * plan_pair(W, Y, num_sms, plan);

@@ -1,4 +1,4 @@
-"""Depths 2 and 3 just below and above the size at which whole-lane grids take
+"""Depths 2 to 4 just below and above the size at which whole-lane grids take
 the K-stage pipeline: the same words as that many one-generation passes."""
 import pytest
 
@@ -7,8 +7,9 @@ import golb200
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("k", [2, 3])
-@pytest.mark.parametrize("words,rows", [(1024, 16384), (1024, 16385), (1023, 16500), (4100, 4100)])
+@pytest.mark.parametrize("k", [2, 3, 4])
+@pytest.mark.parametrize("words,rows", [(1024, 16384), (1024, 16385), (1023, 16500), (4100, 4100),
+                                        (512, 33000), (256, 65536), (256, 65537)])
 def test_equals_single_passes(words, rows, k):
     import torch
     torch.manual_seed(words + k)
