@@ -1024,7 +1024,11 @@ struct gol_batch {
     int rjobs = 0, rctas = 0;
     size_t rsmem = 0;
     golb200::ResidentBatchPlan rplan;
-    uint32_t* h_stage = nullptr;          // pinned: the grid a fetch brings in (the largest so far)
+    // Pinned: the grid that a fetch brings in. One fetch at a time has it
+    // (stage_busy, under stage_mutex); those beside it copy pageable.
+    std::mutex stage_mutex;
+    bool stage_busy = false;
+    uint32_t* h_stage = nullptr;
     size_t stage_words = 0;
     double last_ms = 0;
     std::string err;
@@ -1051,6 +1055,42 @@ constexpr int kRetuneFineRows = 16;        // the planner's smallest band
 // settling variant of the 512-grid workload: 65.2 ms for 3.51 M computed
 // items against 52.5 ms for 3.56 M untracked ones).
 constexpr double kTrackItemCost = 1.25;
+
+// A fetch's hold on the batch's pinned buffer (a copy to pageable memory goes
+// through the CUDA driver's own, a piece at a time): words is null while
+// another thread's fetch has it, or where no pinned memory can be had. The
+// buffer is made once, for the batch's largest grid.
+struct StageLease {
+    gol_batch* b;
+    uint32_t* words = nullptr;
+    StageLease(gol_batch* batch, size_t n) : b(batch) {
+        if (n == 0) return;
+        std::lock_guard<std::mutex> lk(b->stage_mutex);
+        if (b->stage_busy) return;
+        if (n > b->stage_words) {
+            size_t largest = n;
+            for (const auto& e : b->grids) largest = std::max(largest, (size_t)e.W * e.Y);
+            if (b->h_stage) cudaFreeHost(b->h_stage);
+            b->h_stage = nullptr;
+            b->stage_words = 0;
+            if (cudaMallocHost(reinterpret_cast<void**>(&b->h_stage), largest * sizeof(uint32_t)) !=
+                cudaSuccess) {
+                cudaGetLastError();
+                return;
+            }
+            b->stage_words = largest;
+        }
+        b->stage_busy = true;
+        words = b->h_stage;
+    }
+    ~StageLease() {
+        if (!words) return;
+        std::lock_guard<std::mutex> lk(b->stage_mutex);
+        b->stage_busy = false;
+    }
+    StageLease(const StageLease&) = delete;
+    StageLease& operator=(const StageLease&) = delete;
+};
 
 int forced_band(const gol_batch::Entry& e) { return e.force_band ? e.force_band : e.tile_rows_hint; }
 
@@ -1519,20 +1559,10 @@ int gol_batch_fetch(gol_batch* b, int32_t grid_id, uint8_t* cells) {
     auto& e = b->grids[grid_id];
     const int which = e.result_buf;
     const size_t n = (size_t)e.W * e.Y;
-    // Through a pinned buffer (a copy to pageable memory goes through the CUDA
-    // driver's own, a piece at a time); pageable where none can be had.
+    const StageLease lease(b, n);
     std::vector<uint32_t> pageable;
-    if (n > b->stage_words) {
-        if (b->h_stage) cudaFreeHost(b->h_stage);
-        b->h_stage = nullptr;
-        b->stage_words = 0;
-        if (cudaMallocHost(reinterpret_cast<void**>(&b->h_stage), n * sizeof(uint32_t)) == cudaSuccess)
-            b->stage_words = n;
-        else
-            cudaGetLastError();
-    }
-    uint32_t* words = b->h_stage;
-    if (n > b->stage_words) {
+    uint32_t* words = lease.words;
+    if (!words) {
         pageable.resize(n);
         words = pageable.data();
     }
