@@ -532,23 +532,33 @@ int gol_run(gol_engine* e, uint64_t n) {
         return GOL_OK;
     }
     if (budget == 0 && passes >= 2 * (uint64_t)kGraphPasses) {
+        // An even number of passes a chunk: every chunk of the run starts from
+        // e->cur. The graph is built before the grid is touched.
+        if (!e->chunk[e->cur] && (rc = build_chunk_graph(e, e->cur))) return rc;
         // Row-pair passes in chunks run on the grid interleaved (two passes
         // over memory more, a tenth of the integer work of each pass less).
+        // Words outside this block are as they are: a failed launch restores
+        // them too, and if that fails the grid is given up.
+        cudaError_t ce = cudaSuccess;
         if (e->plan.pair) {
-            cudaError_t ce = golb200::launch_interleave(e->d[e->cur], e->W, e->Y, false, e->stream);
+            ce = golb200::launch_interleave(e->d[e->cur], e->W, e->Y, false, e->stream);
             if (ce != cudaSuccess) return e->cuda_fail(ce, "interleave launch");
         }
-        while (passes >= (uint64_t)kGraphPasses) {
-            if (!e->chunk[e->cur] && (rc = build_chunk_graph(e, e->cur))) return rc;
-            cudaError_t ce = cudaGraphLaunch(e->chunk[e->cur], e->stream);
-            if (ce != cudaSuccess) return e->cuda_fail(ce, "graph launch");
+        while (passes >= (uint64_t)kGraphPasses && ce == cudaSuccess) {
+            ce = cudaGraphLaunch(e->chunk[e->cur], e->stream);
+            if (ce != cudaSuccess) break;
             passes -= kGraphPasses;
             e->performed += (uint64_t)kGraphPasses * k;
         }
         if (e->plan.pair) {
-            cudaError_t ce = golb200::launch_interleave(e->d[e->cur], e->W, e->Y, true, e->stream);
-            if (ce != cudaSuccess) return e->cuda_fail(ce, "interleave launch");
+            cudaError_t back = golb200::launch_interleave(e->d[e->cur], e->W, e->Y, true, e->stream);
+            if (back != cudaSuccess) {
+                e->initialized = false;
+                e->has_host_grid = false;
+                return e->cuda_fail(back, "interleave launch (the grid is lost: set the input again)");
+            }
         }
+        if (ce != cudaSuccess) return e->cuda_fail(ce, "graph launch");
     }
     for (; passes > 0; --passes) {
         if (time_is_up()) return GOL_OK;
