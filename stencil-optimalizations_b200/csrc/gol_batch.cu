@@ -743,8 +743,21 @@ struct ResidentDeviceInfo {
 std::mutex g_resident_info_mu;
 std::map<int, ResidentDeviceInfo> g_resident_info;
 
+// Makes `device` the current one for a scope.
+struct DeviceScope {
+    int was = -1;
+    explicit DeviceScope(int device) {
+        if (cudaGetDevice(&was) != cudaSuccess || was == device || cudaSetDevice(device) != cudaSuccess)
+            was = -1;
+    }
+    ~DeviceScope() {
+        if (was >= 0) cudaSetDevice(was);
+    }
+};
+
 const char* resident_device(int device, size_t smem, int* smem_optin, int* per_sm) {
     std::lock_guard<std::mutex> lock(g_resident_info_mu);
+    const DeviceScope scope(device);   // the limit is the current device's
     ResidentDeviceInfo& d = g_resident_info[device];
     if (!d.smem_optin) {
         int v = 0;

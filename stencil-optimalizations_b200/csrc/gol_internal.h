@@ -3,11 +3,26 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 #include <vector>
 
 namespace golb200 {
+
+// Lets a kernel take `bytes` of dynamic shared memory on the current device.
+// The limit is each device's own, so it is raised on every device that the
+// kernel is launched on, once (raised: those it was raised on, a bit each).
+inline cudaError_t raise_smem_limit(const void* kernel, size_t bytes, std::atomic<uint64_t>& raised) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const uint64_t bit = dev < 64 ? 1ull << dev : 0ull;   // (further ones: on every launch)
+    if (raised.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) raised.fetch_or(bit, std::memory_order_relaxed);
+    return e;
+}
 
 // Largest temporal depth instantiated for a given words-per-lane width.
 // The register rings grow as 8 * K * WPL words per thread, so K * WPL <= 16

@@ -28,11 +28,11 @@ namespace {
 template <int WPL, int K>
 cudaError_t launch_one(const RowsLaunch& a, const RowsPlan& p, cudaStream_t stream) {
     // Deep passes need more than the default 48 KB of dynamic shared memory
-    // (the edge table grows with K): opt in once per instantiation.
-    static const cudaError_t attr_ok = cudaFuncSetAttribute(
-        rows_temporal_kernel<WPL, K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-        (int)temporal_smem_bytes(K, kTemporalMaxThreads, WPL));
-    if (attr_ok != cudaSuccess) return attr_ok;
+    // (the edge table grows with K).
+    static std::atomic<uint64_t> raised{0};
+    const cudaError_t e = raise_smem_limit((const void*)rows_temporal_kernel<WPL, K>,
+                                           temporal_smem_bytes(K, kTemporalMaxThreads, WPL), raised);
+    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.nbands, p.nslices);
     cfg.blockDim = dim3(p.threads);
@@ -84,10 +84,10 @@ cudaError_t launch_block(const BlockLaunch& a, cudaStream_t stream) {
 // The row-pair pipeline, a programmatic dependent too.
 template <bool INTER>
 cudaError_t launch_pair(const RowsLaunch& a, const RowsPlan& p, cudaStream_t stream) {
-    static const cudaError_t attr_ok =
-        cudaFuncSetAttribute(rows_pair_kernel<kPairK, INTER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)pair_smem_bytes(kPairK));
-    if (attr_ok != cudaSuccess) return attr_ok;
+    static std::atomic<uint64_t> raised{0};
+    const cudaError_t e = raise_smem_limit((const void*)rows_pair_kernel<kPairK, INTER>,
+                                           pair_smem_bytes(kPairK), raised);
+    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.nbands, p.nslices);
     cfg.blockDim = dim3(p.threads);

@@ -563,16 +563,15 @@ template <int K>
 cudaError_t launch_tracked_one(const RowsLaunch& a, const TileTrack& tt, const int* dense,
                                const RowsPlan& p, int num_sms, cudaStream_t stream) {
     constexpr int WPL = tracked_wpl(K);
-    static const cudaError_t attr_ok = [] {
-        cudaError_t e = cudaFuncSetAttribute(rows_tracked_kernel<WPL, K>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)temporal_smem_bytes(K, kTemporalMaxThreads, WPL, true));
-        return e == cudaSuccess ? set_carveout(rows_tracked_kernel<WPL, K>) : e;
-    }();
-    if (attr_ok != cudaSuccess) return attr_ok;
+    static const cudaError_t carveout_ok = set_carveout(rows_tracked_kernel<WPL, K>);
+    if (carveout_ok != cudaSuccess) return carveout_ok;
+    static std::atomic<uint64_t> raised{0};
+    cudaError_t e = raise_smem_limit((const void*)rows_tracked_kernel<WPL, K>,
+                                     temporal_smem_bytes(K, kTemporalMaxThreads, WPL, true), raised);
+    if (e != cudaSuccess) return e;
     const size_t smem = temporal_smem_bytes(K, p.threads, WPL, true);
     int per_sm = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rows_tracked_kernel<WPL, K>,
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rows_tracked_kernel<WPL, K>,
                                                                   p.threads, smem);
     if (e != cudaSuccess) return e;
     const int units = p.nbands * p.nslices;
