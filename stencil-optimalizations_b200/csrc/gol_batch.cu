@@ -293,14 +293,14 @@ batch_kernel(const BatchGrid* __restrict__ grids, const BatchItem* __restrict__ 
         // every item.
         const int k = it.pass == G.passes - 1 ? G.last_k : G.k;
         if (TRACK && G.trk && k == G.k) {
-            const unsigned still = *(volatile const uint32_t*)(G.trk + 2 * nper);
+            const unsigned still = *(volatile const uint32_t*)G.trk;
             if ((unsigned)(G.pass0 + it.pass) >= still) {   // the grid stopped changing
                 int next = 0;
                 if (lane == 0) {
                     next = atomicAdd(ticket, 1);
                     // every flag from the still pass on is zero; writing this
                     // pass's keeps a later reader from seeing an older one
-                    *(volatile uint32_t*)(G.trk + (((G.parity0 + it.pass) & 1) ? nper : 0) + cell) = 0u;
+                    *(volatile uint32_t*)(G.trk + 1 + (((G.parity0 + it.pass) & 1) ? nper : 0) + cell) = 0u;
                     release_max(mine, it.pass + 1);
                     atomicAdd(G.gstat + 1, 1u);
                     if (G.rflag) *(volatile int*)G.rflag = 1;
@@ -358,8 +358,9 @@ batch_kernel(const BatchGrid* __restrict__ grids, const BatchItem* __restrict__ 
         const long long t_work = clock64();
         const bool odd = (G.parity0 + it.pass) & 1;
         bool compute = true;
-        if (TRACK && G.trk && k == G.k) {   // did the neighbourhood change in the previous pass?
-            const uint32_t* prev = G.trk + (odd ? 0 : nper);   // parity of pass - 1
+        // did the neighbourhood change in the previous pass?
+        if (TRACK && G.trk && k == G.k && (it.pass > 0 || !G.fresh)) {
+            const uint32_t* prev = G.trk + 1 + (odd ? 0 : nper);   // parity of pass - 1
             const uint32_t f = dep >= 0 ? *(volatile const uint32_t*)(prev + dep) : 0u;
             compute = __any_sync(0xffffffffu, f != 0u);
         }
@@ -386,7 +387,7 @@ batch_kernel(const BatchGrid* __restrict__ grids, const BatchItem* __restrict__ 
         const BatchGrid* gp = grids + it.grid;
         uint32_t* trk = TRACK ? ld_ptr_again(&gp->trk) : nullptr;
         if (TRACK && trk && lane == 0)   // this pass's flag, read by the next pass
-            *(volatile uint32_t*)(trk + (odd ? nper : 0) + cell) = (changed || k != G.k) ? 1u : 0u;
+            *(volatile uint32_t*)(trk + 1 + (odd ? nper : 0) + cell) = (changed || k != G.k) ? 1u : 0u;
         // (the release is cumulative over what the warp barrier orders before it)
         if constexpr (!BLOCK) __threadfence();
         __syncwarp();
@@ -405,7 +406,7 @@ batch_kernel(const BatchGrid* __restrict__ grids, const BatchItem* __restrict__ 
                 if (atomicAdd(pstat + 2 * it.pass, 1) == nper - 1) {
                     __threadfence();
                     if (atomicAdd(pstat + 2 * it.pass + 1, 0) == 0) {
-                        atomicMin(trk + 2 * nper, (unsigned)(ld_int_again(&gp->pass0) + it.pass + 1));
+                        atomicMin(trk, (unsigned)(ld_int_again(&gp->pass0) + it.pass + 1));
                         int* rflag = ld_ptr_again(&gp->rflag);
                         if (rflag) *(volatile int*)rflag = 1;
                     }
@@ -1335,7 +1336,7 @@ int gol_batch_upload(gol_batch* b) {
                       (e.auto_track >= 0 ? e.auto_track == 1 : g.passes >= kTrackMinPasses)));
         if (e.tracked) {
             e.trk_offset = trk_words;
-            trk_words += golb200::batch_trk_words(g.ngroups, g.nslices);
+            trk_words += golb200::batch_trk_words((size_t)g.ngroups * g.nslices);
             e.pstat_offset = pstat_words;
             pstat_words += 2 * (size_t)g.passes;
             b->track_any = true;
@@ -1735,7 +1736,7 @@ int gol_batch_grid_stats(gol_batch* b, int32_t grid_id, uint32_t* tracked, uint3
     if (ce == cudaSuccess)
         ce = cudaMemcpy(st, b->d_gstat + 2 * (size_t)grid_id, sizeof(st), cudaMemcpyDeviceToHost);
     if (ce == cudaSuccess && e.tracked)
-        ce = cudaMemcpy(&still, b->d_trk + e.trk_offset + 2 * (size_t)e.choice.ngroups * e.choice.nslices,
+        ce = cudaMemcpy(&still, b->d_trk + e.trk_offset,
                         sizeof(still), cudaMemcpyDeviceToHost);
     if (ce != cudaSuccess) return b->cuda_fail(ce, "batch grid stats");
     if (tracked) *tracked = e.tracked ? 1u : 0u;

@@ -227,20 +227,21 @@ struct BatchGrid {
     // Change tracking (trk null: every item is computed). An item is a tile:
     // it is recomputed only if it or one of its 3x3 neighbour items changed
     // in the previous pass.
-    uint32_t* trk;         // [2][ngroups * nslices] change flags by absolute pass
-                           // parity (parity0 + pass) & 1, nonzero = changed; then one
-                           // word: the pass from which nothing changes (0xFFFFFFFF: none)
+    uint32_t* trk;         // the pass from which nothing changes (0xFFFFFFFF: none), then
+                           // [2][ngroups * nslices] change flags by absolute pass
+                           // parity (parity0 + pass) & 1, nonzero = changed
     int* pstat;            // per pass of this launch: [items done, items changed]
     uint32_t* gstat;       // items computed, items skipped (accumulated)
     int* rflag;            // set to 1 once the grid is known to be still (may be null)
     int pass0;             // passes this grid ran in earlier launches (the still pass
                            // in trk counts from the grid's first launch)
+    int fresh;             // nonzero: the flags say nothing of the pass before (first pass
+                           // of other items than those of the launch before): pass 0
+                           // computes every item
 };
 
-// Words of a grid's change-tracking region (trk).
-inline size_t batch_trk_words(int ngroups, int nslices) {
-    return 2 * (size_t)ngroups * nslices + 1;
-}
+// Words of a grid's change-tracking region (trk): `items` of a pass.
+inline size_t batch_trk_words(size_t items) { return 2 * items + 1; }
 
 struct BatchItem {
     int grid, group, slice, pass;

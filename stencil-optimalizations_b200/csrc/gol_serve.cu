@@ -36,6 +36,13 @@ constexpr int kRoundsInFlight = 3;
 constexpr uint64_t kServeTrackMinPasses = 8;   // auto: requests this long track changes
 constexpr size_t kStageBytes = (size_t)256 << 20;   // pinned staging ring for host inputs
 
+// Band heights that a request's items can have, shortest first. A short band
+// makes a pass's items quick (a pass of 8 generations: 8 rows 4.6 us alone, 48
+// rows 9.2), a tall one computes fewer rows beside its own (2.1 times the work
+// at 8 rows against 48).
+constexpr int kBandCaps = 6;
+constexpr int kBands[kBandCaps] = {8, 12, 16, 24, 32, 48};
+
 struct Request {
     uint64_t id = 0;
     uint64_t x = 0, y = 0;
@@ -51,7 +58,11 @@ struct Request {
     bool tracked = false;       // skips still tiles (its flags live in its slot)
     bool early = false;         // finished before its last planned round: it became still
     int parity = 0;             // buffer holding the state after the rounds queued so far
-    golb200::GridChoice plan{};
+    golb200::GridChoice plan{};   // k for good; the items by the last round's band (0: none yet)
+    struct {
+        int band;               // the cheapest one of up to kBands[cap] rows
+        double cost, crit;      // of one pass (choose_block_plan)
+    } by_cap[kBandCaps];
     int state = 0;              // 0 queued, 1 admitted, 2 finished (after its last round), 3 fetched
     int last_round_slot = -1;   // round buffer slot of its final round
     uint64_t last_round_seq = 0;
@@ -374,24 +385,37 @@ int gol_serve_create(gol_server** out, int32_t device, uint64_t arena_bytes, uin
 
 // Every request runs in the register-block form, whose one kernel body serves
 // every depth and band height (pipelines of several widths in one launch
-// compete for the instruction cache). A round lasts as long as its longest
-// request's chain of passes, so the plan weighs the chain beside the work. A
-// request found still is done at once only where its depth divides its
-// generations, so one that 4 divides and 8 does not takes depth 4.
+// compete for the instruction cache). Its depth is its own for good: 8, and 4
+// where 4 divides its generations and 8 does not (a request found still is done
+// at once only where its depth divides them). Its band is each round's
+// (plan_bands).
 // Its slot in the arena: the two grid buffers, two counters (items computed / skipped)
-// and, when it tracks changes, its change flags and still pass (the
+// and, when it tracks changes, its still pass and change flags (the
 // batch kernel's tracking region), kept for the request's whole life.
 static bool plan_request(gol_server* s, Request& r, uint64_t generations) {
-    if (!golb200::choose_block_plan(r.W, r.Y, std::max<uint64_t>(generations, 1),
-                                    generations % 8 == 4 ? 4 : 0, 0, &r.plan,
-                                    4.0 * s->num_sms, 1.0))
-        return false;
-    const uint64_t passes = (generations + r.plan.k - 1) / r.plan.k;
+    const int k = generations % 8 == 4 || generations <= 4 ? 4 : 8;
+    size_t most = 0;   // items of a pass
+    r.plan = {};
+    for (int c = 0; c < kBandCaps; ++c) {
+        golb200::GridChoice ch;
+        if (c > 0) r.by_cap[c] = r.by_cap[c - 1];
+        if (!golb200::choose_block_plan(r.W, r.Y, (uint64_t)k, k, kBands[c], &ch)) return false;
+        if (c == 0 || ch.cost < r.by_cap[c].cost) {
+            r.by_cap[c].band = kBands[c];
+            r.by_cap[c].cost = ch.cost;
+            r.by_cap[c].crit = ch.crit;
+            most = std::max(most, (size_t)ch.ngroups * ch.nslices);
+        }
+    }
+    r.plan.k = k;
+    const uint64_t passes = (generations + k - 1) / k;
     r.tracked = s->track_mode == GOL_TRACK_ON ||
                 (s->track_mode == GOL_TRACK_AUTO && passes >= kServeTrackMinPasses);
     r.stride = ((size_t)r.W * r.Y + 63) / 64 * 64;
-    const size_t extra = 2 + (r.tracked ? golb200::batch_trk_words(r.plan.ngroups, r.plan.nslices) : 0);
-    r.slot_words = 2 * r.stride + (extra + 63) / 64 * 64;
+    auto slot = [&](size_t extra) { return 2 * r.stride + (2 + extra + 63) / 64 * 64; };
+    // (a request that fills the arena runs without flags)
+    r.tracked = r.tracked && slot(golb200::batch_trk_words(most)) <= s->arena_words;
+    r.slot_words = slot(r.tracked ? golb200::batch_trk_words(most) : 0);
     return true;
 }
 
@@ -411,6 +435,35 @@ static uint64_t round_generations(const gol_server* s, const Request& r) {
     const uint64_t k = (uint64_t)r.plan.k;
     const uint64_t q = std::max(k, s->quantum / k * k);
     return left <= q ? left : q;
+}
+
+// The bands of a round of passes: the tallest allowed (an index into kBands).
+// A round takes about its work over the schedulers and, beside it, its longest
+// chain of dependent passes: few requests want short chains (short bands),
+// many want little work (tall bands), so the cap whose estimate is least is
+// chosen round by round from what is running. Against short bands whatever
+// runs: a stream of 2000 requests a second p50 / p99 8.5 / 125 -> 4.2 / 63 ms
+// (219 -> 91 M items), a burst of 24 requests 14.1 -> 13.5 ms.
+static int plan_bands(gol_server* s) {
+    double work[kBandCaps] = {}, chain[kBandCaps] = {};
+    for (uint64_t id : s->running) {
+        const Request& r = s->reqs[id];
+        const double passes = (double)((round_generations(s, r) + r.plan.k - 1) / r.plan.k);
+        for (int c = 0; c < kBandCaps; ++c) {
+            work[c] += passes * r.by_cap[c].cost;
+            chain[c] = std::max(chain[c], passes * r.by_cap[c].crit);
+        }
+    }
+    int best = 0;
+    double best_time = 0;
+    for (int c = 0; c < kBandCaps; ++c) {
+        const double time = work[c] / (4.0 * s->num_sms) + chain[c];
+        if (c == 0 || time < best_time) {
+            best = c;
+            best_time = time;
+        }
+    }
+    return best;
 }
 
 // A resident round: every running request advances up to the quantum of
@@ -566,13 +619,10 @@ int gol_serve_step(gol_server* s) {
         } else {
             ce = upload_words(s, s->arena + off, r.words);
         }
-        // counters zero; change flags "changed" (the first pass computes
-        // every tile) and no still pass
+        // counters zero and no still pass (the flags are the first round's to write)
         if (ce == cudaSuccess) ce = cudaMemsetAsync(slot_gstat(s, r), 0, 2 * sizeof(uint32_t), s->stream);
         if (ce == cudaSuccess && r.tracked)
-            ce = cudaMemsetAsync(slot_trk(s, r), 0xff,
-                                 golb200::batch_trk_words(r.plan.ngroups, r.plan.nslices) * sizeof(uint32_t),
-                                 s->stream);
+            ce = cudaMemsetAsync(slot_trk(s, r), 0xff, sizeof(uint32_t), s->stream);
         if (ce != cudaSuccess) return s->cuda_fail(ce, "request upload");
         std::vector<uint32_t>().swap(r.words);   // a pageable source is staged before the call returns
         if (r.gens == 0) {               // nothing to run: finished at once
@@ -601,9 +651,15 @@ int gol_serve_step(gol_server* s) {
     std::vector<size_t> pstat_off;   // per grid: its pass counters in rb.d_pstat (tracked grids)
     std::vector<uint64_t> still;
     rb.ids.clear();
+    const int cap = plan_bands(s);
     for (uint64_t id : s->running) {
         Request& r = s->reqs[id];
         const uint64_t g = round_generations(s, r);
+        // Other bands than the last round's are other items: the change flags
+        // then say nothing of them, and the round's first pass computes all.
+        const bool fresh = r.plan.band != r.by_cap[cap].band;
+        if (fresh && !golb200::choose_block_plan(r.W, r.Y, (uint64_t)r.plan.k, r.plan.k, r.by_cap[cap].band, &r.plan))
+            return s->fail(GOL_E_UNSUPPORTED, "no plan for this request");
         golb200::GridChoice ch = r.plan;
         ch.passes = (int)((g + ch.k - 1) / ch.k);
         ch.last_k = g % ch.k ? (int)(g % ch.k) : ch.k;
@@ -616,6 +672,7 @@ int gol_serve_step(gol_server* s) {
         bg.done_base = done;
         done += bg.ngroups * bg.nslices;
         max_passes = std::max(max_passes, bg.passes);
+        bg.fresh = fresh;
         bg.gstat = slot_gstat(s, r);
         pstat_off.push_back(pstat);
         if (r.tracked) {   // flags and still pass stay in the slot between rounds
