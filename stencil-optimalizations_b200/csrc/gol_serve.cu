@@ -386,14 +386,14 @@ int gol_serve_create(gol_server** out, int32_t device, uint64_t arena_bytes, uin
 // Every request runs in the register-block form, whose one kernel body serves
 // every depth and band height (pipelines of several widths in one launch
 // compete for the instruction cache). Its depth is its own for good: 8, and 4
-// where 4 divides its generations and 8 does not (a request found still is done
-// at once only where its depth divides them). Its band is each round's
-// (plan_bands).
+// where a round's quantum is under 8 generations, or where 4 divides its
+// generations and 8 does not (a request found still is done at once only where
+// its depth divides them). Its band is each round's (plan_bands).
 // Its slot in the arena: the two grid buffers, two counters (items computed / skipped)
 // and, when it tracks changes, its still pass and change flags (the
 // batch kernel's tracking region), kept for the request's whole life.
 static bool plan_request(gol_server* s, Request& r, uint64_t generations) {
-    const int k = generations % 8 == 4 || generations <= 4 ? 4 : 8;
+    const int k = s->quantum < 8 || generations % 8 == 4 || generations <= 4 ? 4 : 8;
     size_t most = 0;   // items of a pass
     r.plan = {};
     for (int c = 0; c < kBandCaps; ++c) {
