@@ -80,7 +80,9 @@
 
 namespace golb200 {
 
-constexpr long long kSpinLimit = 1ll << 24;   // polls of >= 64 ns: a few-second guard
+// A wait gives up after this many polls, of 64 ns and a round trip to L2 each
+// (about 13 s in all); a longer sleep counts as the polls it stands for.
+constexpr long long kSpinLimit = 1ll << 24;
 
 namespace {
 
@@ -336,7 +338,7 @@ batch_kernel(const BatchGrid* __restrict__ grids, const BatchItem* __restrict__ 
                 // ahead do not crowd the counters (a lone 2048^2 grid: 14.2 us
                 // a pass with all of them polling).
                 const unsigned ns = behind > 1 ? 1000u * min(behind - 1, 64) : 64u;
-                spins += ns / 64;
+                spins += 1 + ns / 1024;
                 if (__any_sync(0xffffffffu, spins > spin_limit || *(volatile int*)status != 0)) {
                     if (lane == 0) atomicCAS(status, 0, GOL_E_TIMEOUT);
                     return;
