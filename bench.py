@@ -311,16 +311,6 @@ def run_reference_arm(args, d: Dist) -> None:
 # our arm
 # ---------------------------------------------------------------------------
 
-def pass_kernel(plan: dict, k: int) -> str:
-    """The kernel that the engine's passes of k generations run (no forced
-    band or lane width), by its plan."""
-    if k == 1:
-        return f"rows_once_kernel<{plan['words_per_lane']}>"
-    if plan["words_per_lane"] == 1:
-        return f"rows_block_kernel,{k}"
-    return f"rows_pair_kernel<{k}>"
-
-
 def measured_peaks() -> dict:
     try:
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
@@ -486,7 +476,7 @@ def bench_hbm(stream, device) -> dict:
                         "hbm_frac": gbs / hbm_peak,
                         "int_frac": cu * ALG_INT_OPS_PER_CELL / int_peak,
                         "words_per_lane": plan["words_per_lane"], "band_rows": plan["band_rows"],
-                        "kernel": pass_kernel(plan, k)}
+                        "kernel": golb200.rows_pass_kernel(size, size, k)}
     # parity: every depth gives the k = 1 grid after 96 generations, and
     # k = 1 equals the oracle
     chk = 96
@@ -896,7 +886,7 @@ def run_ours(args, d: Dist) -> None:
     pass_cell_updates = size * size * best_k
     int_achieved = pass_cell_updates * ALG_INT_OPS_PER_CELL / (launch_ms * 1e-3)
     e.close()
-    kernel = pass_kernel(plan, best_k)
+    kernel = golb200.rows_pass_kernel(size, size, best_k)
     hbm_view = {"bound": "hbm", "achieved": achieved_gbs, "peak": hbm_peak, "unit": "GB/s",
                 "frac": achieved_gbs / hbm_peak, "peak_source": peak_src,
                 "algorithmic_bytes_per_launch": alg_bytes,

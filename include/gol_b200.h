@@ -274,6 +274,12 @@ int gol_rows_pass(const void* d_src, void* d_dst, uint64_t x, uint64_t y, uint32
  * then runs the K-stage kernel). */
 int gol_rows_pass_ex(const void* d_src, void* d_dst, uint64_t x, uint64_t y, uint32_t k,
                      uint32_t band_rows, uint32_t lane_words, void* stream);
+/* The kernel that such a pass runs on the current device, with its template
+ * parameters ("rows_block_kernel<96>"), into name (size bytes, ended by a
+ * zero); GOL_E_UNSUPPORTED where the pass is. An engine's passes of k
+ * generations run the same one. */
+int gol_rows_pass_kernel(uint64_t x, uint64_t y, uint32_t k, uint32_t band_rows,
+                         uint32_t lane_words, char* name, uint32_t size);
 
 /* No counterpart in the reference (its algorithms always cudaMalloc their own
  * grids in initialize_data_structures). For callers that cannot allocate

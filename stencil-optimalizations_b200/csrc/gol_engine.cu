@@ -706,6 +706,31 @@ int gol_rows_pass_ex(const void* d_src, void* d_dst, uint64_t x, uint64_t y, uin
     return ce == cudaSuccess ? GOL_OK : GOL_E_CUDA;
 }
 
+int gol_rows_pass_kernel(uint64_t x, uint64_t y, uint32_t k, uint32_t band_rows,
+                         uint32_t lane_words, char* name, uint32_t size) {
+    if (!name || !size || x % 32 || k < 1 || k > (uint32_t)golb200::kMaxTemporalSteps ||
+        x / 32 > (uint64_t)1 << 30 || y > (uint64_t)1 << 30)
+        return GOL_E_INVALID;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        cudaGetLastError();
+        dev = 0;
+    }
+    RowsPlan p;
+    if (!golb200::plan_rows((int)(x / 32), (int)y, (int)k, (int)band_rows, (int)lane_words,
+                            golb200::device_sm_count(dev), &p))
+        return GOL_E_UNSUPPORTED;
+    if (p.block)
+        std::snprintf(name, size, "rows_block_kernel<%d>", p.block);
+    else if (p.pair)
+        std::snprintf(name, size, "rows_pair_kernel<%u>", k);
+    else if (p.stream)
+        std::snprintf(name, size, "rows_%s_kernel<%d>", p.once ? "once" : "stream", p.wpl);
+    else
+        std::snprintf(name, size, "rows_temporal_kernel<%d,%u>", p.wpl, k);
+    return GOL_OK;
+}
+
 int gol_pack_cells_device(const uint8_t* d_cells, void* d_words, uint64_t x, uint64_t y,
                           void* stream) {
     if ((!d_cells || !d_words) && x * y) return GOL_E_INVALID;

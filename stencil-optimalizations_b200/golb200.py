@@ -117,6 +117,7 @@ def lib():
     L.gol_plan.argtypes = [_vp, ctypes.POINTER(_u32), ctypes.POINTER(_u32), ctypes.POINTER(_u32)]
     L.gol_rows_pass.argtypes = [_vp, _vp, _u64, _u64, _u32, _u32, _vp]
     L.gol_rows_pass_ex.argtypes = [_vp, _vp, _u64, _u64, _u32, _u32, _u32, _vp]
+    L.gol_rows_pass_kernel.argtypes = [_u64, _u64, _u32, _u32, _u32, ctypes.c_char_p, _u32]
     L.gol_pack_cells_device.argtypes = [_vp, _vp, _u64, _u64, _vp]
     L.gol_unpack_cells_device.argtypes = [_vp, _vp, _u64, _u64, _vp]
     L.gol_load_random_ones_zeros.argtypes = [_vp, _u64, _u64, _u64]
@@ -523,6 +524,15 @@ def rows_pass(d_src: int, d_dst: int, x: int, y: int, k: int, band_rows: int = 0
     rc = lib().gol_rows_pass_ex(d_src, d_dst, x, y, k, band_rows, lane_words, stream)
     if rc != GOL_OK:
         raise RuntimeError(f"gol_rows_pass failed with status {rc}")
+
+
+def rows_pass_kernel(x: int, y: int, k: int, band_rows: int = 0, lane_words: int = 0) -> str:
+    """The kernel that rows_pass, or an engine's passes of k generations, run."""
+    name = ctypes.create_string_buffer(64)
+    rc = lib().gol_rows_pass_kernel(x, y, k, band_rows, lane_words, name, len(name))
+    if rc != GOL_OK:
+        raise RuntimeError(f"gol_rows_pass_kernel failed with status {rc}")
+    return name.value.decode()
 
 
 def pack_cells_device(d_cells: int, d_words: int, x: int, y: int, stream: int = 0) -> None:
