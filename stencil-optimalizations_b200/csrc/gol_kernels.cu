@@ -200,12 +200,108 @@ static double plan_pair(int W, int Y, int num_sms, RowsPlan* p) {
     return best;
 }
 
+// CTAs per SM that the K-stage pipeline's bands are cut for.
+static int stage_ctas_per_sm(int warps) { return warps >= 4 ? 2 : 2 * ((4 + warps - 1) / warps); }
+
+// The K-stage pipeline's CTAs (p->wpl words per lane).
+static void plan_stage(int W, int Y, int k, int band_rows, int num_sms, RowsPlan* p) {
+    const int wpl = p->wpl, lanes = W / wpl;
+    if (lanes <= kTemporalMaxThreads) {
+        p->slice = W;
+        p->nslices = 1;
+        p->halo = 0;
+        p->threads = std::max(32, (lanes + 31) / 32 * 32);
+    } else {
+        const int per = kTemporalMaxThreads - 2;               // one halo lane each side
+        const int ns = (lanes + per - 1) / per;
+        const int slice_lanes = (lanes + ns - 1) / ns;
+        p->slice = slice_lanes * wpl;
+        p->nslices = (W + p->slice - 1) / p->slice;
+        p->halo = wpl;
+        p->threads = (slice_lanes + 2 + 31) / 32 * 32;
+    }
+    int band = band_rows;
+    if (band <= 0) {
+        // About two CTAs per SM, or more when a CTA has fewer than four
+        // warps (narrow grids: at 8192^2, k = 4, 2-warp CTAs with 16-row
+        // bands ran at 18.9 T cell-updates/s against 16.0 T with 28-row
+        // ones); never thinner than a few times the depth, whose y-halo
+        // costs ~k extra rows per stage per band.
+        const int per_sm = stage_ctas_per_sm(p->threads / 32);
+        const int target = std::max(1, per_sm * num_sms / p->nslices);
+        band = (Y + target - 1) / target;
+        band = std::max(band, std::max(8, 4 * k));
+    }
+    band = std::min(band, std::max(Y, 1));
+    p->band = band;
+    p->nbands = (Y + band - 1) / band;
+}
+
+// How many times as fast as the other forms the K-stage pipeline with geometry
+// p is at a pass of k generations, where it is the fastest (0 elsewhere).
+// On grids whose two buffers fill L2 or more it can be: it reads
+// each row about once, the blocks of 30 columns their halos again, and CTAs of
+// whole warps waste nothing. What it gains over the register blocks there
+// depends on the words per lane, the depth and the warps per CTA, and falls
+// with the share of its threads that own words (part; whole: rows of whole
+// warps, which start on a line) and by the halo lanes of slices. Some pay only
+// where the CTAs fill every SM alike, most of these with no short band among
+// them: the next pass's CTAs, let in early, land unevenly otherwise. Measured
+// from 24 to 256 MiB a buffer, us a pass, pipeline / blocks: 32768^2 64 / 74 and
+// 88 / 97 (k = 2, 3), 32640 x 32768 67 / 74 and 30720 x 32768 66 / 71 (k = 2),
+// 16384 x 65536 68 / 79 (k = 2; at k = 3, a short last band, 118 / 103),
+// 4096 x 262144 114 / 158 and 8192 x 65536 57 / 72 (k = 4), 7936 x 67650 60 / 68
+// (k = 4); in L2 the blocks win: 16384 x 12288 18 / 16 (k = 2).
+static double stage_gain(const RowsPlan& p, int W, int Y, int k, int num_sms) {
+    enum Fill { kAny, kEven, kNoShort };
+    struct Gain {
+        int wpl, k, warps;
+        Fill fill;
+        int words;   // least size of the grid, 2^20 words
+        double whole, part;
+    };
+    static constexpr Gain kGains[] = {
+        {4, 2, 1, kAny, 15, 1.14, 1.14},     {4, 2, 2, kNoShort, 15, 1.25, 1.25},
+        {4, 2, 4, kEven, 15, 1.16, 1.13},    {4, 2, 6, kAny, 18, 1.02, 0.0},
+        {4, 2, 7, kAny, 15, 1.05, 0.0},      {4, 2, 8, kAny, 15, 1.15, 1.13},
+        {4, 3, 1, kAny, 12, 1.07, 1.25},
+        {4, 3, 4, kNoShort, 12, 1.18, 1.13}, {4, 3, 8, kAny, 12, 1.09, 1.04},
+        {4, 4, 1, kAny, 12, 1.35, 1.24},     {4, 4, 2, kAny, 8, 1.30, 1.20},
+        {2, 5, 1, kAny, 12, 1.15, 0.0},      {2, 5, 4, kNoShort, 12, 1.05, 0.0},
+        {2, 6, 1, kAny, 12, 1.10, 0.0},      {2, 6, 2, kAny, 8, 1.18, 1.08},
+        {2, 6, 4, kNoShort, 12, 1.03, 0.0},  {2, 7, 1, kAny, 12, 1.15, 0.0},
+        {2, 7, 2, kAny, 8, 1.18, 1.08},      {2, 7, 4, kAny, 12, 1.05, 0.0},
+        {2, 8, 2, kAny, 32, 1.05, 0.0},      {2, 8, 4, kAny, 16, 1.05, 0.0},
+        {1, 15, 4, kAny, 24, 1.04, 0.0},     {1, 16, 4, kAny, 16, 1.04, 0.0},
+    };
+    const int warps = p.threads / 32, lanes = p.slice / p.wpl;
+    const bool even = (long long)p.nbands * p.nslices == (long long)stage_ctas_per_sm(warps) * num_sms;
+    const bool no_short = even && 3ll * (Y - (p.nbands - 1) * p.band) >= p.band;
+    for (const Gain& g : kGains) {
+        if (g.wpl != p.wpl || g.k != k || g.warps != warps) continue;
+        if ((long long)W * Y < (long long)g.words << 20) return 0;
+        if (g.fill == kEven ? !even : g.fill == kNoShort && !no_short) return 0;
+        const double gain =
+            (p.nslices > 1 ? 0.95 : 1.0) * (lanes == p.threads ? g.whole : g.part * lanes / p.threads);
+        return gain > 1.015 ? gain : 0;
+    }
+    return 0;
+}
+
 // The depth at which a generation costs least, a tie going to the row-pair
-// pipeline (its interleaved passes against the register-block ones).
+// pipeline (its interleaved passes against the register-block ones). Tall
+// narrow grids on which the K-stage pipeline beats the blocks at depth 4 by
+// more than they gain from 4 to 8 (1.2 times) take it: 4096 x 131072 15.6 us a
+// generation against 17.2 at depth 8, 8192 x 65536 14.0 against 15.1.
 int best_depth(int W, int Y, int num_sms) {
     int best = 4;
     double t = 0;
-    RowsPlan pair;
+    RowsPlan pair, stage;
+    if (W % 4 == 0 && W > 0) {
+        stage.wpl = 4;
+        plan_stage(W, Y, 4, 0, num_sms, &stage);
+        if (stage_gain(stage, W, Y, 4, num_sms) > 1.2) return 4;
+    }
     for (int k : {4, 6, 8, 12, 16}) {
         const double u = best_block(W, std::max(Y, 1), k, num_sms).us / k;
         if (t == 0 || u < t) {
@@ -216,8 +312,6 @@ int best_depth(int W, int Y, int num_sms) {
     const double u = plan_pair(W, Y, num_sms, &pair) / kPairK;
     return u > 0 && u <= t ? kPairK : best;
 }
-
-constexpr long long kStageWords = 16 << 20;   // 64 MiB a buffer
 
 bool plan_rows(int W, int Y, int k, int band_rows, int wpl, int num_sms, RowsPlan* plan,
                bool k_stage) {
@@ -240,35 +334,6 @@ bool plan_rows(int W, int Y, int k, int band_rows, int wpl, int num_sms, RowsPla
     plan->stream = k == 1 && !k_stage;
     plan->block = 0;
     plan->pair = false;
-    // Grids whose two buffers fill L2 or more, in one slice of whole warps: the
-    // K-stage pipeline reads each row about once, the blocks of 30 columns
-    // their halos again. Pipeline against the other kernels, us a pass:
-    // 32768^2 64 / 75 and 88 / 96 (k = 2, 3), 16384 x 65536 68 / 78 (k = 2, but
-    // 119 / 102 at k = 3), 24576^2 45 / 45 and 63 / 59, 8192 x 65536 57 / 72 at
-    // k = 4 and 48 / 46 at k = 2; in several slices 65536 x 16384 88 / 73, and
-    // in L2 16384^2 25 / 20.
-    const int lanes4 = W / 4;
-    const bool stages = wpl == 4 && (long long)W * Y >= kStageWords && lanes4 % 32 == 0 &&
-                        lanes4 <= kTemporalMaxThreads &&
-                        ((k == 2 && lanes4 >= 128) || (k == 3 && lanes4 > 224) ||
-                         (k == kPairK && lanes4 <= 64));
-    if (k > 1 && !k_stage && !forced && !stages) {
-        const BlockChoice c = best_block(W, std::max(Y, 1), k, num_sms);
-        if (k == kPairK) {   // rows as they are take the pipeline an eighth longer
-            const double us = 1.13 * plan_pair(W, Y, num_sms, plan);
-            if (us > 0 && us <= c.us) return true;
-            plan->pair = false;
-        }
-        plan->wpl = 1;
-        plan->threads = 32;
-        plan->block = c.R;
-        plan->band = c.B;
-        plan->nbands = (int)(((long long)Y + c.B - 1) / c.B);
-        plan->slice = kBlockOwn;
-        plan->nslices = (W + kBlockOwn - 1) / kBlockOwn;
-        plan->halo = 1;
-        return true;
-    }
     if (plan->stream) {
         // One generation: lanes of wpl words across the row, each thread
         // loading its short band whole, or with a forced band walking that.
@@ -283,36 +348,23 @@ bool plan_rows(int W, int Y, int k, int band_rows, int wpl, int num_sms, RowsPla
         plan->nbands = (Y + band - 1) / band;
         return true;
     }
-    if (lanes <= kTemporalMaxThreads) {
-        plan->slice = W;
-        plan->nslices = 1;
-        plan->halo = 0;
-        plan->threads = std::max(32, (lanes + 31) / 32 * 32);
-    } else {
-        const int per = kTemporalMaxThreads - 2;               // one halo lane each side
-        const int ns = (lanes + per - 1) / per;
-        const int slice_lanes = (lanes + ns - 1) / ns;
-        plan->slice = slice_lanes * wpl;
-        plan->nslices = (W + plan->slice - 1) / plan->slice;
-        plan->halo = wpl;
-        plan->threads = (slice_lanes + 2 + 31) / 32 * 32;
+    plan_stage(W, Y, k, band_rows, num_sms, plan);
+    if (k > 1 && !k_stage && !forced && stage_gain(*plan, W, Y, k, num_sms) == 0) {
+        const BlockChoice c = best_block(W, std::max(Y, 1), k, num_sms);
+        if (k == kPairK) {   // rows as they are take the pipeline an eighth longer
+            const double us = 1.13 * plan_pair(W, Y, num_sms, plan);
+            if (us > 0 && us <= c.us) return true;
+            plan->pair = false;
+        }
+        plan->wpl = 1;
+        plan->threads = 32;
+        plan->block = c.R;
+        plan->band = c.B;
+        plan->nbands = (int)(((long long)Y + c.B - 1) / c.B);
+        plan->slice = kBlockOwn;
+        plan->nslices = (W + kBlockOwn - 1) / kBlockOwn;
+        plan->halo = 1;
     }
-    int band = band_rows;
-    if (band <= 0) {
-        // About two CTAs per SM, or more when a CTA has fewer than four
-        // warps (narrow grids: at 8192^2, k = 4, 2-warp CTAs with 16-row
-        // bands ran at 18.9 T cell-updates/s against 16.0 T with 28-row
-        // ones); never thinner than a few times the depth, whose y-halo
-        // costs ~k extra rows per stage per band.
-        const int warps = plan->threads / 32;
-        const int per_sm = warps >= 4 ? 2 : 2 * ((4 + warps - 1) / warps);
-        const int target = std::max(1, per_sm * num_sms / plan->nslices);
-        band = (Y + target - 1) / target;
-        band = std::max(band, std::max(8, 4 * k));
-    }
-    band = std::min(band, std::max(Y, 1));
-    plan->band = band;
-    plan->nbands = (Y + band - 1) / band;
     return true;
 }
 

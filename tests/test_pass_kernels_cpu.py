@@ -19,6 +19,32 @@ def test_kernel_by_name(x, y, k, band, lanes, kernel):
     assert golb200.rows_pass_kernel(x, y, k, band, lanes) == kernel
 
 
+@pytest.mark.parametrize("x,y,k,kernel", [
+    # large grids next to 32768 and 8192 cells wide, where the K-stage pipeline
+    # is the faster form too
+    (32640, 32768, 2, "rows_temporal_kernel<4,2>"),
+    (30720, 32768, 2, "rows_temporal_kernel<4,2>"),
+    (32640, 32768, 3, "rows_temporal_kernel<4,3>"),
+    (65024, 16384, 2, "rows_temporal_kernel<4,2>"),
+    (8192, 65536, 4, "rows_temporal_kernel<4,4>"),
+    (7936, 67650, 4, "rows_temporal_kernel<4,4>"),
+    (3840, 200000, 4, "rows_temporal_kernel<4,4>"),
+    (4096, 262144, 7, "rows_temporal_kernel<2,7>"),
+    # and where it is not: warps that do not share the SMs evenly, idle lanes, L2
+    (20480, 32768, 2, "rows_block"),
+    (18432, 32768, 3, "rows_block"),
+    (33280, 32768, 2, "rows_block"),
+    (6144, 131072, 4, "rows_block"),
+    (16384, 12288, 2, "rows_block"),
+])
+def test_large_grids(x, y, k, kernel):
+    got = golb200.rows_pass_kernel(x, y, k)
+    if kernel == "rows_block":
+        assert got.startswith(kernel)
+    else:
+        assert got == kernel
+
+
 def test_refused():
     for args in ((64, 64, 17), (48, 64, 1), (96, 64, 2, 0, 4)):
         with pytest.raises(RuntimeError):
