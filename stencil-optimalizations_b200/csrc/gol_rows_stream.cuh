@@ -184,7 +184,7 @@ rows_stream_kernel(RowsLaunch a) {
 // of a plain copy) where the walk took 48.8, 16384^2 9.3 against 12.3. Bands of
 // 6 / 8 / 12 / 16 rows in CTAs of 128 ran 32768^2 in 46.1 / 44.1 / 43.4 / 43.8 us,
 // 16 rows in CTAs of 64 in 43.1.
-constexpr int kOnceThreads = 64;
+constexpr int kOnceThreads = 64;   // at most (32 for rows of an odd number of warps)
 template <int WPL>
 __host__ __device__ constexpr int once_rows() { return WPL == 4 ? 16 : WPL == 2 ? 16 : 30; }
 

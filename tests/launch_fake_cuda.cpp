@@ -78,6 +78,12 @@ cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 int main() {
     using namespace golb200;
     alignas(16) static uint32_t a[4], b[4];   // (never read or written)
+    // One-generation passes: a row's CTAs have no warp past its end.
+    for (int lanes : {1, 31, 32, 33, 64, 65, 96, 97, 128, 160, 224, 256, 257}) {
+        RowsPlan p;
+        CHECK(plan_rows(4 * lanes, 1000, 1, 0, 0, 148, &p) && p.once && p.threads <= 64);
+        CHECK(p.nslices * p.threads == (lanes + 31) / 32 * 32);
+    }
     for (int round = 0; round < 2; ++round) {
         for (int dev = 0; dev < 3; ++dev) {
             current = dev;
