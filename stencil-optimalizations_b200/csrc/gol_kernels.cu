@@ -378,12 +378,34 @@ bool plan_rows(int W, int Y, int k, int band_rows, int wpl, int num_sms, RowsPla
 #define GOL_RESIDENT_THREADS 512   // threads per CTA (lanes across a row x row groups)
 #endif
 
-#ifndef GOL_RESIDENT_ROWS
-// Row groups are cut so that each has about this many rows or more (a group
-// reads two rows beside its own): 1 / 2 / 3 ran 1024 generations of 2048^2 in
-// 0.79 / 0.82 / 0.75 ms, of 3072 x 1024 in 0.84 / 0.80 / 0.99 ms.
-#define GOL_RESIDENT_ROWS 2
-#endif
+// Row groups of a resident run's CTA (bands of `band` rows of `lanes` lanes). A
+// generation is a chain (barrier, row loads, the thread's rows) on narrow
+// bands, and integer work of the fullest scheduler on wide ones. Measured over
+// 100 shapes, every count of groups, us per 1024 generations:
+//   under 16 lanes a row a group, up to 256 threads or so (544 x 700: 824 with
+//   two rows a group, 698 so; 512^2 747, 630), with 8 lanes half of them on
+//   short bands (bank conflicts between the groups of a warp: 1024 x 4096 811,
+//   748);
+//   16 lanes, rows of whole half-warps and wide rows: counts that load the four
+//   schedulers alike (2048^2 784 with 11 groups, 757 with 8; 12288 x 1024 1447
+//   with 5, 1366 with 4; 4096^2 1030 with 16, 943 with 8; 8192 x 1024 1025 with
+//   8, 960 with 4; 8192^2 1948 with 8, 1978 with 4, 1927 with 6);
+//   others two rows or more a group, up to the CTA's threads.
+static int resident_groups(int lanes, int band, int K) {
+    const int most = std::min(GOL_RESIDENT_THREADS, kResidentMaxThreads) / lanes;
+    int n = (band + K + 1) / 2;
+    if (lanes < 16) {
+        n = std::min(lanes > 12 ? 20 : std::min(32, 256 / lanes), band + 2 * K);
+        if (lanes == 8 && band < 40) n = std::min(n, 16);
+    } else if (lanes == 16) {
+        n = band < 20 ? 8 : 20;
+    } else if (lanes > 80 && lanes <= 112) {
+        n = 4;
+    } else if (lanes % 16 == 0 && lanes >= 32 && lanes <= 80) {
+        n = lanes < 64 ? 8 : band < 28 ? 4 : 6;
+    }
+    return std::max(1, std::min(n, most));
+}
 
 bool plan_resident(int W, int Y, int k_epoch, int device, ResidentPlan* p) {
     const int K = k_epoch > 0 ? k_epoch : GOL_RESIDENT_K;
@@ -408,8 +430,7 @@ bool plan_resident(int W, int Y, int k_epoch, int device, ResidentPlan* p) {
     if (2ull * (band + 2 * K) * accepted * sizeof(uint32_t) + 1024 > (size_t)smem_max) return false;
     const size_t smem = resident_smem_bytes(band, K, lanes);
     p->lanes = lanes;
-    p->groups = std::max(1, std::min(std::min(GOL_RESIDENT_THREADS, kResidentMaxThreads) / lanes,
-                                     (band + K + GOL_RESIDENT_ROWS - 1) / GOL_RESIDENT_ROWS));
+    p->groups = resident_groups(lanes, band, K);
     p->K = K;
     p->band = band;
     p->nbands = nbands;
