@@ -969,6 +969,7 @@ void fill_resident_jobs(const ResidentBatchPlan& p, const ResidentGrid* g, unsig
             j.b = band;
             j.nb = pg.nb;
             j.gens = e.gens;
+            j.epoch0 = 0;   // (the slots are zeroed before each launch)
         }
     }
 }

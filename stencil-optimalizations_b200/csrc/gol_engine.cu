@@ -56,6 +56,7 @@ struct gol_engine {
     bool resident = false;
     golb200::ResidentPlan rplan{};
     unsigned long long* r_pub = nullptr;   // exchange slots
+    int r_epochs = 0;                      // epochs run on them so far
     int* r_status = nullptr;
 
     // change tracking (GOL_ALG_LOCAL)
@@ -110,6 +111,7 @@ void release_device(gol_engine* e) {
     if (e->r_pub) cudaFree(e->r_pub);
     if (e->r_status) cudaFree(e->r_status);
     e->r_pub = nullptr;
+    e->r_epochs = 0;
     e->r_status = nullptr;
     for (auto& p : e->d) {
         if (p) cudaFree(p);
@@ -483,8 +485,8 @@ int gol_run(gol_engine* e, uint64_t n) {
             if (time_is_up()) return GOL_OK;
             const uint64_t chunk = std::min<uint64_t>(n - done, budget ? step : (1ull << 30));
             cudaError_t ce = golb200::launch_resident(e->d[e->cur], e->d[e->cur ^ 1], e->W, e->Y,
-                                                      (long long)chunk, e->rplan, e->r_pub, e->r_status,
-                                                      e->stream);
+                                                      (long long)chunk, e->rplan, e->r_pub, &e->r_epochs,
+                                                      e->r_status, e->stream);
             if (ce == cudaSuccess && budget) ce = cudaStreamSynchronize(e->stream);
             if (ce != cudaSuccess) return e->cuda_fail(ce, "resident run launch");
             e->cur ^= 1;

@@ -66,7 +66,7 @@ int best_depth(int W, int Y, int num_sms);
 struct ResidentBand {
     const uint32_t* src;   // the grid at generation 0 (row r at src + r * pitch)
     uint32_t* dst;         // the grid after `gens` generations (not src)
-    unsigned long long* pub;   // the grid's exchange slots, zero at start: band b's at (b * 4 + parity * 2 + side)
+    unsigned long long* pub;   // the grid's exchange slots, tags up to epoch0: band b's at (b * 4 + parity * 2 + side)
                            // * K * 4 * lanes words (side 0: its top K rows, 1: its bottom K rows)
     int pitch;             // words from one grid row to the next (>= W)
     int W, Y;              // words per row, rows
@@ -74,6 +74,7 @@ struct ResidentBand {
     int lanes, groups;     // threads: lanes of four words across a row x row groups
     int b, nb;             // this band, bands of the grid (rows split evenly)
     long long gens;
+    int epoch0;            // number of the first epoch (epoch e's tag is e + 1)
 };
 
 // A grid of a resident batch launch (batch_resident_kernel).
@@ -122,11 +123,12 @@ struct ResidentPlan {
 // False when the grid does not fit (or k_epoch is out of range). k_epoch = 0
 // picks the default.
 bool plan_resident(int W, int Y, int k_epoch, int device, ResidentPlan* p);
-// gens generations src -> dst. pub (p.pub_words) and status are device
-// scratch, cleared here.
+// gens generations src -> dst. pub (p.pub_words) and status are device scratch;
+// *epochs_done counts the epochs of the launches on pub (0: none yet, pub is
+// cleared here).
 cudaError_t launch_resident(const uint32_t* src, uint32_t* dst, int W, int Y, long long gens,
-                            const ResidentPlan& p, unsigned long long* pub, int* status,
-                            cudaStream_t stream, long long spin_limit = 0);
+                            const ResidentPlan& p, unsigned long long* pub, int* epochs_done,
+                            int* status, cudaStream_t stream, long long spin_limit = 0);
 
 // Row-pair passes can run on grids interleaved by four (interleaved below),
 // which launch_interleave does in place (back: undoes). Rows of whole lanes

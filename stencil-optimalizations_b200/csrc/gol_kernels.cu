@@ -1,6 +1,7 @@
 // Kernel instantiations and launch dispatch for the row-band temporal
 // kernel, plus device-side pack/unpack between uint8 cells and row words.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 
 #include "gol_b200.h"
@@ -454,13 +455,26 @@ static cudaError_t launch_resident_lanes(const ResidentLaunch& a, const Resident
 }
 
 cudaError_t launch_resident(const uint32_t* src, uint32_t* dst, int W, int Y, long long gens,
-                            const ResidentPlan& p, unsigned long long* pub, int* status,
-                            cudaStream_t stream, long long spin_limit) {
-    cudaError_t e = cudaMemsetAsync(pub, 0, p.pub_words * sizeof(unsigned long long), stream);
+                            const ResidentPlan& p, unsigned long long* pub, int* epochs_done,
+                            int* status, cudaStream_t stream, long long spin_limit) {
+    const long long epochs = (gens + p.K - 1) / p.K;
+    int epoch0 = *epochs_done;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(stream, &capture);
+    // Slots never used, numbers about to run out, or a launch that may be
+    // replayed: from zero. (A replay leaves tags up to its epochs, which later
+    // launches count on from.)
+    const bool full = epoch0 + epochs >= INT_MAX;
+    if (epoch0 == 0 || full || capture != cudaStreamCaptureStatusNone) {
+        if (e == cudaSuccess) e = cudaMemsetAsync(pub, 0, p.pub_words * sizeof(unsigned long long), stream);
+        if (full) *epochs_done = 0;
+        epoch0 = 0;
+    }
     if (e == cudaSuccess) e = cudaMemsetAsync(status, 0, sizeof(int), stream);
     if (e != cudaSuccess) return e;
+    *epochs_done = std::max(*epochs_done, (int)(epoch0 + epochs));
     ResidentLaunch a{src, dst, pub, status, W, Y, p.K, p.lanes, p.groups, gens,
-                     spin_limit > 0 ? spin_limit : (1ll << 24)};
+                     spin_limit > 0 ? spin_limit : (1ll << 24), epoch0};
     // Rows of 4096, 8192 and 16384 cells get a compile-time row stride.
     switch (p.lanes) {
         case 32: return launch_resident_lanes<32>(a, p, stream);

@@ -24,8 +24,9 @@
 // Epoch e publishes the band's top and bottom K rows into slot e & 1, every
 // word with the epoch's tag e + 1 beside it in one 64-bit store: the
 // neighbours poll the words themselves, so an exchange costs one trip through
-// L2 and no fence, counter or barrier of its own (the slots are zeroed before
-// a launch). A CTA rewrites a slot two epochs later, after both neighbours
+// L2 and no fence, counter or barrier of its own. Launches on the same slots
+// count their epochs on, so that no tag comes twice (a memset of the slots
+// before each took 3 to 6 us). A CTA rewrites a slot two epochs later, after both neighbours
 // have published the epoch in between, i.e. after they read it.
 //
 // Within a pass a thread owns four words of a row (128 cells; the CTA's
@@ -74,7 +75,7 @@ constexpr int kResidentInterior = GOL_RESIDENT_INTERIOR;
 struct ResidentLaunch {   // one grid (rows_resident_kernel)
     const uint32_t* src;   // the grid at generation 0 (W words per row, Y rows)
     uint32_t* dst;         // the grid after `gens` generations (not src)
-    unsigned long long* pub;   // [nbands][2 parities][2 sides][K rows][4 planes][lanes], zero at launch
+    unsigned long long* pub;   // [nbands][2 parities][2 sides][K rows][4 planes][lanes], tags up to epoch0
     int* status;           // GOL_E_TIMEOUT if a wait gave up
     int W, Y;
     int K;                 // generations per epoch
@@ -82,6 +83,7 @@ struct ResidentLaunch {   // one grid (rows_resident_kernel)
     int groups;            // row groups (blockDim.x = lanes * groups)
     long long gens;
     long long spin_limit;
+    int epoch0;            // number of the launch's first epoch
 };
 
 // A published word: the value below, the epoch's tag above, stored and loaded
@@ -348,7 +350,7 @@ __device__ __forceinline__ bool resident_band(const ResidentBand& j, uint32_t* s
 
     int cur = 0;
     long long left = j.gens;
-    for (int e = 0; left > 0; ++e) {
+    for (int e = j.epoch0; left > 0; ++e) {
         const int kk = (int)min((long long)K, left);
         // Publish the band's top and bottom K rows (the state at epoch start).
         const uint32_t tag = (uint32_t)e + 1u;
@@ -471,6 +473,7 @@ __global__ void __launch_bounds__(kResidentMaxThreads, 1) rows_resident_kernel(R
     j.b = blockIdx.x;
     j.nb = gridDim.x;
     j.gens = a.gens;
+    j.epoch0 = a.epoch0;
     resident_band<LANES>(j, smem, &stop, a.status, a.spin_limit);
 }
 

@@ -46,6 +46,7 @@ cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cu
     std::memcpy(d, s, n);
     return cudaSuccess;
 }
+cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { std::memset(d, v, n); return cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = reinterpret_cast<cudaStream_t>(8); return cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
@@ -99,7 +100,7 @@ void host_copy(void* d, const void* s, size_t n) { std::memcpy(d, s, n); }
 // never reached by a dense run
 bool plan_resident(int, int, int, int, ResidentPlan*) { std::abort(); }
 cudaError_t launch_resident(const uint32_t*, uint32_t*, int, int, long long, const ResidentPlan&,
-                            unsigned long long*, int*, cudaStream_t, long long) { std::abort(); }
+                            unsigned long long*, int*, int*, cudaStream_t, long long) { std::abort(); }
 bool plan_local_tiles(int, int, int, int, int, int, int, LocalPlan*) { std::abort(); }
 cudaError_t launch_local_pass(const uint32_t*, uint32_t*, int, int, int, const LocalPlan&,
                               const LocalState&, int, cudaStream_t) { std::abort(); }

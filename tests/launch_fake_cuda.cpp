@@ -56,6 +56,7 @@ cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const
     *n = 1;
     return cudaSuccess;
 }
+cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* s) { *s = cudaStreamCaptureStatusNone; return cudaSuccess; }
 cudaError_t cudaPeekAtLastError() { return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void*, int, size_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaMalloc(void**, size_t) { return cudaErrorMemoryAllocation; }
