@@ -356,7 +356,7 @@ int gol_set_input_words(gol_engine* e, const void* words, uint64_t x, uint64_t y
     int rc = check_shape(e, x, y);
     if (rc) return rc;
     if ((rc = ensure_host(e))) return rc;
-    golb200::host_copy(e->h_words, words, e->h_bytes);   // same bytes for 32- and 64-bit rows
+    golb200::host_copy(e->h_words, words, e->h_bytes, true);   // same bytes for 32- and 64-bit rows
     e->has_host_grid = true;
     e->performed = 0;
     return GOL_OK;
@@ -631,7 +631,7 @@ int gol_fetch_words(gol_engine* e, void* words, uint32_t word_bits) {
     if (e->x % word_bits) return e->fail(GOL_E_INVALID, "x must be a multiple of word_bits");
     if (!e->has_host_grid || e->initialized) return e->fail(GOL_E_STATE, "fetch before finalize");
     if (!words && e->h_bytes) return e->fail(GOL_E_INVALID, "null words");
-    golb200::host_copy(words, e->h_words, e->h_bytes);
+    golb200::host_copy(words, e->h_words, e->h_bytes, false);
     return GOL_OK;
 }
 

@@ -179,12 +179,26 @@ void parallel_rows(size_t y, size_t bytes_per_row, F&& body) {
 
 } // namespace
 
-void host_copy(void* dst, const void* src, size_t bytes) {
+void host_copy(void* dst, const void* src, size_t bytes, bool for_device) {
     // by pages, so that the ranges' first touches of dst are spread too
     constexpr size_t kPage = 4096;
     parallel_rows((bytes + kPage - 1) / kPage, kPage, [=](size_t p0, size_t p1) {
         const size_t a = p0 * kPage, b = std::min(bytes, p1 * kPage);
-        std::memcpy(static_cast<char*>(dst) + a, static_cast<const char*>(src) + a, b - a);
+        char* d = static_cast<char*>(dst) + a;
+        const char* s = static_cast<const char*>(src) + a;
+#ifdef GOL_HAVE_STREAM_STORES
+        if (for_device && (reinterpret_cast<uintptr_t>(d) & 15u) == 0) {
+            size_t i = 0;
+            for (; i + 64 <= b - a; i += 64)
+                for (size_t j = 0; j < 64; j += 16)
+                    _mm_stream_si128(reinterpret_cast<__m128i*>(d + i + j),
+                                     _mm_loadu_si128(reinterpret_cast<const __m128i*>(s + i + j)));
+            std::memcpy(d + i, s + i, b - a - i);
+            _mm_sfence();
+            return;
+        }
+#endif
+        std::memcpy(d, s, b - a);
     });
 }
 

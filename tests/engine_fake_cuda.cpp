@@ -95,7 +95,7 @@ cudaError_t launch_interleave(uint32_t* grid, int W, int Y, bool back, cudaStrea
     enqueue([=] { for (int i = 0; i < W * Y; ++i) grid[i] ^= kInter; });
     return cudaSuccess;
 }
-void host_copy(void* d, const void* s, size_t n) { std::memcpy(d, s, n); }
+void host_copy(void* d, const void* s, size_t n, bool) { std::memcpy(d, s, n); }
 
 // never reached by a dense run
 bool plan_resident(int, int, int, int, ResidentPlan*) { std::abort(); }
