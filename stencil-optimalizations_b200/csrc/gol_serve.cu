@@ -113,6 +113,7 @@ struct gol_server {
     };
     std::deque<StageUse> stage_uses;       // uploads whose staging bytes may still be read
     std::vector<cudaEvent_t> free_events;
+    cudaEvent_t slots_free = nullptr;      // the rounds that still touch a freed slot
     int num_sms = 148;
     uint32_t* arena = nullptr;
     size_t arena_words = 0;
@@ -264,6 +265,22 @@ cudaError_t upload_words(gol_server* s, uint32_t* dst, const std::vector<uint32_
     }
     s->stage_uses.push_back({pos, len, ev});
     s->stage_head = pos + len;
+    return cudaSuccess;
+}
+
+// Returns a finished request's slot to the arena. Rounds queued before the
+// request was found still have items of it left; those end at once, but they
+// count themselves and zero its flags: uploads (on their own stream) into the
+// slot wait for the rounds queued so far.
+cudaError_t free_slot(gol_server* s, const Request& r) {
+    if (r.early) {
+        cudaError_t ce = cudaSuccess;
+        if (!s->slots_free) ce = cudaEventCreateWithFlags(&s->slots_free, cudaEventDisableTiming);
+        if (ce == cudaSuccess) ce = cudaEventRecord(s->slots_free, s->stream);
+        if (ce == cudaSuccess) ce = cudaStreamWaitEvent(s->upload_stream, s->slots_free, 0);
+        if (ce != cudaSuccess) return ce;
+    }
+    arena_free(s, r.offset, r.slot_words);
     return cudaSuccess;
 }
 
@@ -765,7 +782,7 @@ int gol_serve_fetch(gol_server* s, uint64_t id, uint8_t* cells) {
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(s->copy_stream);
     if (ce != cudaSuccess) return s->cuda_fail(ce, "result copy");
     golb200::host_unpack_u8(words.data(), r.x, r.y, cells);
-    arena_free(s, r.offset, r.slot_words);
+    if ((ce = free_slot(s, r)) != cudaSuccess) return s->cuda_fail(ce, "slot release");
     s->reqs.erase(it);
     return GOL_OK;
 }
@@ -784,7 +801,7 @@ int gol_serve_fetch_words(gol_server* s, uint64_t id, void* words) {
                              (size_t)r.W * r.Y * sizeof(uint32_t), cudaMemcpyDeviceToHost, s->copy_stream);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(s->copy_stream);
     if (ce != cudaSuccess) return s->cuda_fail(ce, "result copy");
-    arena_free(s, r.offset, r.slot_words);
+    if ((ce = free_slot(s, r)) != cudaSuccess) return s->cuda_fail(ce, "slot release");
     s->reqs.erase(it);
     return GOL_OK;
 }
@@ -795,7 +812,8 @@ int gol_serve_release(gol_server* s, uint64_t id) {
     auto it = s->reqs.find(id);
     if (it == s->reqs.end()) return s->fail(GOL_E_INVALID, "unknown request");
     if (it->second.state != 2) return s->fail(GOL_E_STATE, "request not finished");
-    arena_free(s, it->second.offset, it->second.slot_words);
+    const cudaError_t ce = free_slot(s, it->second);
+    if (ce != cudaSuccess) return s->cuda_fail(ce, "slot release");
     s->reqs.erase(it);
     return GOL_OK;
 }
@@ -889,6 +907,7 @@ void gol_serve_destroy(gol_server* s) {
     if (s->d_census) cudaFree(s->d_census);
     if (s->copy_stream) cudaStreamDestroy(s->copy_stream);
     if (s->upload_stream) cudaStreamSynchronize(s->upload_stream);
+    if (s->slots_free) cudaEventDestroy(s->slots_free);
     for (auto& u : s->stage_uses) cudaEventDestroy(u.done);
     for (auto ev : s->free_events) cudaEventDestroy(ev);
     if (s->upload_stream) cudaStreamDestroy(s->upload_stream);
