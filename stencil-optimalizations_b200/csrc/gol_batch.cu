@@ -241,7 +241,8 @@ __device__ __forceinline__ void release_max(int* p, int v) {
 // and instruction footprint are that family's); 0 dispatches on each grid's
 // own width. Warps of one SM that run different bodies compete for the
 // instruction cache, which halved throughput in measurements, so the
-// planner gives a batch one width and one depth.
+// planner gives a batch of pipelines one width and one depth. BLOCK: every
+// grid in the register-block form, whose one body serves all of them.
 //
 // TRACK: grids with a change-tracking region (G.trk) skip the items whose
 // 3x3 neighbour items did not change in the previous pass, the rule of the
@@ -450,7 +451,8 @@ batch_resident_kernel(const ResidentBand* __restrict__ jobs, int njobs, int* tic
 } // namespace
 
 // ---------------------------------------------------------------------------
-// Autotuner: one (words per lane, depth) for the whole batch, a band height
+// Autotuner of the pipeline form (forced lane widths; choose_block_plan below
+// has the others): one (words per lane, depth) for the whole batch, a band height
 // per grid.
 //
 // Model, in units of one word through one stage on a 4-word lane: a work

@@ -49,7 +49,7 @@ struct RowsPlan {
 // Picks words-per-lane and CTA shape for a W-word by Y-row grid and depth k.
 // wpl = 0 chooses the widest lane access whose rings fit k; 1, 2 or 4 forces
 // it. Returns false for k outside 1..16 or a wpl that W or k rules out.
-// k = 1 plans the streaming kernel (band_rows = rows per thread, 0 = auto)
+// k = 1 plans the one-generation kernels (band_rows = rows per thread, 0 = auto)
 // and deeper passes without a forced band or wpl the register-block kernel
 // unless k_stage is set (callers that need the K-stage geometry).
 bool plan_rows(int W, int Y, int k, int band_rows, int wpl, int num_sms, RowsPlan* plan,
