@@ -447,6 +447,8 @@ int gol_init(gol_engine* e) {
     if (e->resident && !e->r_pub) {
         ce = cudaMalloc(&e->r_pub, std::max<size_t>(e->rplan.pub_words, 1) * sizeof(unsigned long long));
         if (ce == cudaSuccess) ce = cudaMalloc(&e->r_status, sizeof(int));
+        if (ce == cudaSuccess)
+            ce = cudaMemsetAsync(e->r_pub, 0, e->rplan.pub_words * sizeof(unsigned long long), e->stream);
         if (ce != cudaSuccess) {
             release_device(e);
             return e->cuda_fail(ce, "resident-run scratch");

@@ -124,8 +124,8 @@ struct ResidentPlan {
 // picks the default.
 bool plan_resident(int W, int Y, int k_epoch, int device, ResidentPlan* p);
 // gens generations src -> dst. pub (p.pub_words) and status are device scratch;
-// *epochs_done counts the epochs of the launches on pub (0: none yet, pub is
-// cleared here).
+// *epochs_done counts the epochs of the launches on pub (0, and pub zeroed,
+// before the first).
 cudaError_t launch_resident(const uint32_t* src, uint32_t* dst, int W, int Y, long long gens,
                             const ResidentPlan& p, unsigned long long* pub, int* epochs_done,
                             int* status, cudaStream_t stream, long long spin_limit = 0);

@@ -461,11 +461,10 @@ cudaError_t launch_resident(const uint32_t* src, uint32_t* dst, int W, int Y, lo
     int epoch0 = *epochs_done;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     cudaError_t e = cudaStreamIsCapturing(stream, &capture);
-    // Slots never used, numbers about to run out, or a launch that may be
-    // replayed: from zero. (A replay leaves tags up to its epochs, which later
-    // launches count on from.)
+    // Numbers about to run out, or a launch that may be replayed: from zero. (A
+    // replay leaves tags up to its epochs, which later launches count on from.)
     const bool full = epoch0 + epochs >= INT_MAX;
-    if (epoch0 == 0 || full || capture != cudaStreamCaptureStatusNone) {
+    if (full || capture != cudaStreamCaptureStatusNone) {
         if (e == cudaSuccess) e = cudaMemsetAsync(pub, 0, p.pub_words * sizeof(unsigned long long), stream);
         if (full) *epochs_done = 0;
         epoch0 = 0;

@@ -82,3 +82,38 @@ def test_captured_and_replayed():
         e.finalize_data_structures()
         # the capture itself ran nothing
         assert np.array_equal(e.fetch_result(), oracle.life_cells(cells, 40 + 6 * n + 5 * n + 2 * n + 2 * n))
+
+
+@pytest.mark.parametrize("replays", [0, 2])
+def test_first_run_captured(replays):
+    """An engine whose first run is only captured, on memory that another
+    engine's slots were in."""
+    torch = pytest.importorskip("torch")
+    x, y = 1056, 400
+    cells = oracle.random_ones_zeros(x, y, 6)
+    s = torch.cuda.Stream()
+
+    def engine():
+        return golb200.GolB200(grid_dimensions=(x, y), state_bits_count=32, algorithm="resident",
+                               stream=s.cuda_stream)
+
+    with engine() as e:
+        e.set_and_format_input_data(cells)
+        e.initialize_data_structures()
+        e.run(200)
+        e.finalize_data_structures()
+    with engine() as e:
+        e.set_and_format_input_data(cells)
+        e.initialize_data_structures()
+        e.sync()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            e.run(50)
+            e.run(50)
+        with torch.cuda.stream(s):
+            for _ in range(replays):
+                graph.replay()
+        e.run(9)
+        e.run(70)
+        e.finalize_data_structures()
+        assert np.array_equal(e.fetch_result(), oracle.life_cells(cells, 100 * replays + 79))
