@@ -277,7 +277,7 @@ int gol_rows_pass_ex(const void* d_src, void* d_dst, uint64_t x, uint64_t y, uin
 /* The kernel that such a pass runs on the current device, with its template
  * parameters ("rows_block_kernel<96>"), into name (size bytes, ended by a
  * zero); GOL_E_UNSUPPORTED where the pass is. An engine's passes of k
- * generations run the same one. */
+ * generations run the same one (thread_block_size as band_rows). */
 int gol_rows_pass_kernel(uint64_t x, uint64_t y, uint32_t k, uint32_t band_rows,
                          uint32_t lane_words, char* name, uint32_t size);
 
